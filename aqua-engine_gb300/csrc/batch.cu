@@ -360,8 +360,8 @@ static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::ve
     for (const DevScene& sc : scenes) full = full || sc.mext != nullptr;
     bool qbvh = false;  // some scene walks quantized nodes
     for (const DevScene& sc : scenes) qbvh = qbvh || sc.qbvh != 0;
-    auto kernel = full ? (qbvh ? k_batch<true, kNodesAny> : k_batch<true, kNodesFull>)
-                       : (qbvh ? k_batch<false, kNodesAny> : k_batch<false, kNodesFull>);
+    auto kernel = full ? (qbvh ? k_batch<true, kNodesOwn> : k_batch<true, kNodesFull>)
+                       : (qbvh ? k_batch<false, kNodesOwn> : k_batch<false, kNodesFull>);
     int per_sm = tune.blocks_per_sm;
     if (per_sm <= 0) {
         AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));

@@ -104,6 +104,10 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     for (const aqua_material& m : h.mats)
         if (m.specular_tint > 0.0f || m.sheen > 0.0f || m.clearcoat > 0.0f || m.transmission > 0.0f) full_bsdf = true;
     size_t total = align256(o_mext + (full_bsdf ? 32 * h.mats.size() : 0));
+    // Walk nodes follow the uploaded image; the device derives them.
+    bool use_walk = !use_q && nn >= kWalkNodesFrom && !ctx->host_only;
+    for (int a = 0; a < 3; ++a)  // a walk node's frame must stay within the float range
+        use_walk = use_walk && std::fabs(s->bvh.lo[a]) < 1e15f && std::fabs(s->bvh.hi[a]) < 1e15f;
     free_staging(s);
     if (ctx->host_only) {
         s->pinned = malloc(total);
@@ -179,10 +183,11 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     s->bvh_format_used = use_q ? AQUA_BVH_QUANTIZED : AQUA_BVH_FULL;
     if (ctx->host_only) return;  // host-only context: no device image
     dev_free(s->dev);
-    dev_alloc(ctx, s->dev, total);
+    dev_alloc(ctx, s->dev, total + (use_walk ? sizeof(float) * kBvhQNodeFloats * nn : 0));
     char* d = (char*)s->dev.ptr;
     DevScene& ds = s->ds;
     ds.nodes = (const float4*)(d + o_nodes);
+    ds.wnodes = use_walk ? (const float4*)(d + total) : nullptr;
     ds.qbvh = use_q ? 1 : 0;
     ds.tris = (const float4*)(d + o_tris);
     ds.uvs = (const float2*)(d + o_uvs);
@@ -200,6 +205,7 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     for (int i = 0; i < 3; ++i) ds.env[i] = h.env[i];
     ds.cam = dev_camera(h.cam);
     scene_upload(ctx, s);
+    if (use_walk) build_walk_nodes(ctx, ds, (float4*)(d + total));
 }
 
 void scene_upload(aqua_ctx* ctx, aqua_scene* s) {

@@ -239,6 +239,15 @@ struct aqua_ctx {
 
 namespace aq {
 
+// Trees of at least this many nodes are walked through walk nodes. A smaller
+// tree's full-precision nodes are served by L1 and L2 well enough that the
+// walk is bound by instruction issue, and the tighter boxes win; rooms of
+// tessellated spheres, 512 x 512 at 16 spp and 1M random rays, full against
+// walk nodes: 8 nodes (Cornell GGX 1024^2, 64 spp) 38.4 / 45.2 ms; 6.0k nodes
+// 3.57 / 3.77 ms and 188 / 192 us; 33k 4.32 / 4.41 ms and 228 / 231 us; 131k
+// 4.82 / 4.87 ms and 260 / 252 us; the interior's 294k 47.9 / 40.8 ms.
+constexpr size_t kWalkNodesFrom = 150000;
+
 // Device allocation through the context (honours the fail_alloc_after hook).
 void dev_alloc(aqua_ctx* ctx, DevBuf& b, size_t bytes);
 void dev_free(DevBuf& b);
@@ -252,6 +261,13 @@ void dev_free(DevBuf& b);
 // where the tree's memory footprint matters.
 constexpr size_t kQuantizeAbove = (size_t)8 << 30;
 void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh = true);
+// Walk nodes (device.cuh, load_walk) of the scene's full-precision nodes:
+// 64 bytes per node, written on the context's stream.
+void build_walk_nodes(aqua_ctx* ctx, const DevScene& S, float4* out);
+// The node format a scene's rays walk (kNodes*).
+inline int walk_format(const DevScene& S) {
+    return S.wnodes ? kNodesWalk : S.qbvh ? kNodesQuantized : kNodesFull;
+}
 void scene_upload(aqua_ctx* ctx, aqua_scene* s);
 void scene_release(aqua_scene* s);
 DevCamera dev_camera(const aqua_camera& c);

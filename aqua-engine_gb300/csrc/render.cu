@@ -225,7 +225,7 @@ __device__ __forceinline__ void ltrain_add(float4* L, uint32_t id, v3 c) {
     L[id] = v;
 }
 
-template <bool SORTED, bool COUNT>
+template <bool SORTED, bool COUNT, int NODES>
 __global__ void __launch_bounds__(128) k_trace_ext(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
                                                    uint32_t cnt_out) {
     grid_dep_wait();
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(128) k_trace_ext(DevScene S, WaveParams P, Wav
     };
     if (!COUNT) {
         // Persistent lanes with ray replacement.
-        traverse_queue<false>(
+        traverse_queue<kQueueClosest, NODES>(
             S, n, &W.counters[kCntFetchTrace],
             [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
                 uint32_t s = W.q_in[i];
@@ -591,7 +591,7 @@ __device__ __forceinline__ void shadow_done(const WaveParams& P, const WavePtrs&
     }
 }
 
-template <bool COUNT, bool NRC = false>
+template <bool COUNT, bool NRC, int NODES>
 __global__ void __launch_bounds__(128) k_shadow(DevScene S, WaveParams P, WavePtrs W) {
     grid_dep_wait();
     grid_dep_launch();
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(128) k_shadow(DevScene S, WaveParams P, WavePt
     uint32_t nodes = 0, tris = 0;
     auto finish = [&](uint32_t i, const TraceResult& r) { shadow_done<NRC>(P, W, i, r); };
     if (!COUNT) {
-        traverse_queue<true>(
+        traverse_queue<kQueueAny, NODES>(
             S, n, &W.counters[kCntFetchShadow],
             [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
                 float4 ro = W.sh_o[i], rd = W.sh_d[i];
@@ -648,7 +648,7 @@ __global__ void __launch_bounds__(128) k_shadow(DevScene S, WaveParams P, WavePt
 // fills (cnt_out, sh_out). Film updates keep their order per slot: a
 // slot's shadow contribution of bounce k lands before bounce k + 1 is
 // shaded, as in the three-launch pipeline.
-template <bool NRC = false>
+template <bool NRC, int NODES>
 __global__ void __launch_bounds__(128) k_trace_fused(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
                                                      uint32_t cnt_out, uint32_t sh_in, uint32_t sh_out) {
     grid_dep_wait();
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(128) k_trace_fused(DevScene S, WaveParams P, W
         W.counters[sh_out] = 0;
     }
     constexpr uint32_t kShadowTag = 0x80000000u;
-    traverse_queue_kind<kQueueMixed>(
+    traverse_queue<kQueueMixed, NODES>(
         S, n_ext + n_sh, &W.counters[kCntFetchTrace],
         [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax, bool& any) -> uint32_t {
             if (i < n_ext) {
@@ -750,6 +750,36 @@ static void ensure_workspace(aqua_ctx* ctx, size_t slots, size_t buckets, size_t
 void workspace_release(aqua_ctx* ctx) {
     dev_free(ctx->ws.block);
     ctx->ws = Workspace{};
+}
+
+// The traversal kernels of a scene's node format (the counting ones walk the
+// canonical tree, whatever the format).
+using TraceKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t);
+using ShadowKernel = void (*)(DevScene, WaveParams, WavePtrs);
+using FusedKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t, uint32_t, uint32_t);
+
+static TraceKernel trace_kernel(const DevScene& S, bool sorted, bool count) {
+    static constexpr TraceKernel walks[2][3] = {
+        {k_trace_ext<false, false, kNodesFull>, k_trace_ext<false, false, kNodesQuantized>,
+         k_trace_ext<false, false, kNodesWalk>},
+        {k_trace_ext<true, false, kNodesFull>, k_trace_ext<true, false, kNodesQuantized>,
+         k_trace_ext<true, false, kNodesWalk>}};
+    if (count) return sorted ? k_trace_ext<true, true, kNodesFull> : k_trace_ext<false, true, kNodesFull>;
+    return walks[sorted][walk_format(S)];
+}
+
+static ShadowKernel shadow_kernel(const DevScene& S, bool count, bool nrc) {
+    static constexpr ShadowKernel walks[2][3] = {
+        {k_shadow<false, false, kNodesFull>, k_shadow<false, false, kNodesQuantized>,
+         k_shadow<false, false, kNodesWalk>},
+        {k_shadow<false, true, kNodesFull>, k_shadow<false, true, kNodesQuantized>, k_shadow<false, true, kNodesWalk>}};
+    return count ? k_shadow<true, false, kNodesFull> : walks[nrc][walk_format(S)];
+}
+
+static FusedKernel fused_kernel(const DevScene& S) {
+    static constexpr FusedKernel walks[3] = {k_trace_fused<true, kNodesFull>, k_trace_fused<true, kNodesQuantized>,
+                                             k_trace_fused<true, kNodesWalk>};
+    return walks[walk_format(S)];
 }
 
 template <class K>
@@ -890,12 +920,11 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     if (bt != 128 && bt != 64 && bt != 32) throw Error(AQUA_ERR_INVALID_ARG, "block_trace must be 32, 64 or 128");
     if (bs != 128 && bs != 64 && bs != 32) throw Error(AQUA_ERR_INVALID_ARG, "block_shade must be 32, 64 or 128");
 
-    auto trace_k = sorted ? (count ? k_trace_ext<true, true> : k_trace_ext<true, false>)
-                          : (count ? k_trace_ext<false, true> : k_trace_ext<false, false>);
+    const TraceKernel trace_k = trace_kernel(S, sorted, count);
     const bool full = S.mext != nullptr;  // some material sets the full model's lobes
     auto shade_k = full ? (sorted ? k_shade<true, false, true> : k_shade<false, false, true>)
                         : (sorted ? k_shade<true> : k_shade<false>);
-    auto shadow_k = count ? k_shadow<true> : k_shadow<false>;
+    const ShadowKernel shadow_k = shadow_kernel(S, count, false);
     int g_trace = grid_for(ctx, trace_k, bt, tune.blocks_per_sm);
     int g_shade = grid_for(ctx, shade_k, bs, tune.blocks_per_sm);
     int g_shadow = grid_for(ctx, shadow_k, bt, tune.blocks_per_sm);
@@ -1174,10 +1203,10 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     W.q_pix = nw.q_pix; W.q_raw = nw.q_raw; W.rec = nw.rec; W.ltrain = nw.ltrain; W.lsnap = nw.lsnap;
     W.spread = nw.spread;
 
-    auto trace_k = sorted ? k_trace_ext<true, false> : k_trace_ext<false, false>;
+    const TraceKernel trace_k = trace_kernel(S, sorted, false);
     auto shade_k = S.mext ? (sorted ? k_shade<true, true, true> : k_shade<false, true, true>)
                           : (sorted ? k_shade<true, true> : k_shade<false, true>);
-    auto shadow_k = k_shadow<false, true>;
+    const ShadowKernel shadow_k = shadow_kernel(S, false, true);
     int g_trace = grid_for(ctx, trace_k, 128, tune.blocks_per_sm);
     int g_shade = grid_for(ctx, shade_k, 128, tune.blocks_per_sm);
     int g_shadow = grid_for(ctx, shadow_k, 128, tune.blocks_per_sm);
@@ -1189,7 +1218,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     // the 1080p interior). Deep plain renders stay on three launches, where
     // the fused launch measured 2.3% slower (Cornell GGX 1024^2).
     const bool fused = !sorted;
-    auto fused_k = k_trace_fused<true>;
+    const FusedKernel fused_k = fused_kernel(S);
     int g_fused = fused ? grid_for(ctx, fused_k, 128, tune.blocks_per_sm) : 0;
 
     cudaEvent_t ev[4];
@@ -1434,9 +1463,9 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
     AQ_CUDA(cudaMemsetAsync(W.counters, 0, 4 * kNoAllocCounters, st));
     AQ_CUDA(cudaMemsetAsync(W.stats, 0, 8 * kNoAllocStats, st));
 
-    auto trace_k = k_trace_ext<false, false>;
+    const TraceKernel trace_k = trace_kernel(S, false, false);
     auto shade_k = S.mext ? k_shade<false, false, true> : k_shade<false>;
-    auto shadow_k = k_shadow<false>;
+    const ShadowKernel shadow_k = shadow_kernel(S, false, false);
     int g_trace = grid_for(ctx, trace_k, 128, 0);
     int g_shade = grid_for(ctx, shade_k, 128, 0);
     int g_shadow = grid_for(ctx, shadow_k, 128, 0);

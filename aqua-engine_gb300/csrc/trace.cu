@@ -8,7 +8,7 @@
 
 namespace aq {
 
-template <bool ANY, bool COUNT>
+template <bool ANY, bool COUNT, int NODES>
 __global__ void __launch_bounds__(128) k_trace_user(DevScene S, const float4* __restrict__ rays, size_t n,
                                                     float4* __restrict__ hits, unsigned long long* stats) {
     uint32_t nodes = 0, tris = 0;
@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(128) k_trace_user(DevScene S, const float4* __
     if (!COUNT && n < (1ull << 31)) {
         // The renderer's traversal: persistent lanes with ray replacement;
         // stats[2] is the queue cursor.
-        traverse_queue<ANY>(
+        traverse_queue<ANY ? kQueueAny : kQueueClosest, NODES>(
             S, (uint32_t)n, reinterpret_cast<uint32_t*>(stats + 2),
             [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
                 float4 a = ldg_(rays + 2 * (size_t)i), b = ldg_(rays + 2 * (size_t)i + 1);
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128) k_trace_user(DevScene S, const float4* __
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float4 a = ldg_(rays + 2 * i), b = ldg_(rays + 2 * i + 1);
         store(i, COUNT ? traverse<ANY, true>(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, nodes, tris)
-                       : traverse_fast(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, ANY));
+                       : traverse_fast<kNodesOwn>(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, ANY));
     }
     if (COUNT) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -50,6 +50,56 @@ __global__ void __launch_bounds__(128) k_trace_user(DevScene S, const float4* __
             atomicAdd(&stats[1], (unsigned long long)tris);
         }
     }
+}
+
+// One thread per node: the walk node of full-precision node k. All steps
+// are exact: a plane lo + q 2^e of floats lo and 8-bit q needs at most 41
+// bits (2^e is at least an 256th of an ulp of the larger plane), so the
+// doubles below hold it.
+__global__ void k_walk_nodes(const float4* __restrict__ nodes, int32_t n, float4* __restrict__ out) {
+    const int32_t k = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k >= n) return;
+    const float* w = reinterpret_cast<const float*>(nodes + 8 * (size_t)k);
+    const int32_t* link = reinterpret_cast<const int32_t*>(w + 24);
+    float org[3], step[3];
+    uint32_t lo_bytes[3] = {0, 0, 0}, hi_bytes[3] = {0, 0, 0};
+    for (int a = 0; a < 3; ++a) {
+        float lo = INFINITY, hi = -INFINITY;
+        for (int c = 0; c < 4; ++c)
+            if (link[c] != ~0) {
+                lo = fminf(lo, w[8 * a + c]);
+                hi = fmaxf(hi, w[8 * a + 4 + c]);
+            }
+        if (!(lo <= hi)) lo = hi = 0.0f;  // no children (not produced by the builder)
+        int e = -100;
+        if (hi > lo) {  // smallest step whose 255 multiples reach hi
+            e = max(-100, ilogb(((double)hi - (double)lo) / 255.0));
+            if (ldexp(255.0, e) < (double)hi - (double)lo) ++e;
+        }
+        const double s = ldexp(1.0, e);
+        org[a] = lo;
+        step[a] = (float)ldexp(1.0, e + 15);
+        for (int c = 0; c < 4; ++c) {
+            uint32_t ql = 255, qh = 0;  // empty slot: a box no ray enters
+            if (link[c] != ~0) {
+                ql = (uint32_t)floor(((double)w[8 * a + c] - (double)lo) / s);
+                qh = (uint32_t)ceil(((double)w[8 * a + 4 + c] - (double)lo) / s);
+            }
+            lo_bytes[a] |= ql << (8 * c);
+            hi_bytes[a] |= qh << (8 * c);
+        }
+    }
+    float4* o = out + 4 * (size_t)k;
+    o[0] = make_float4(org[0], org[1], org[2], step[0]);
+    o[1] = nodes[8 * (size_t)k + 6];
+    o[2] = make_float4(__uint_as_float(lo_bytes[0]), __uint_as_float(hi_bytes[0]), __uint_as_float(lo_bytes[1]),
+                       __uint_as_float(hi_bytes[1]));
+    o[3] = make_float4(__uint_as_float(lo_bytes[2]), __uint_as_float(hi_bytes[2]), step[1], step[2]);
+}
+
+void build_walk_nodes(aqua_ctx* ctx, const DevScene& S, float4* out) {
+    k_walk_nodes<<<(S.n_nodes + 127) / 128, 128, 0, ctx->stream>>>(S.nodes, S.n_nodes, out);
+    AQ_CUDA(cudaGetLastError());
 }
 
 void trace_rays(aqua_ctx* ctx, aqua_scene* sc, const aqua_ray* rays, size_t n, aqua_hit* out, uint32_t flags,
@@ -79,8 +129,14 @@ void trace_rays(aqua_ctx* ctx, aqua_scene* sc, const aqua_ray* rays, size_t n, a
     if (!ctx->trace_stats.ptr) dev_alloc(ctx, ctx->trace_stats, 64);
     unsigned long long* d_stats = (unsigned long long*)ctx->trace_stats.ptr;
     AQ_CUDA(cudaMemsetAsync(d_stats, 0, 24, st));  // node and triangle counters, queue cursor
-    auto k = any ? (count ? k_trace_user<true, true> : k_trace_user<true, false>)
-                 : (count ? k_trace_user<false, true> : k_trace_user<false, false>);
+    using Kernel = void (*)(DevScene, const float4*, size_t, float4*, unsigned long long*);
+    static constexpr Kernel walks[2][3] = {  // by any, walk_format
+        {k_trace_user<false, false, kNodesFull>, k_trace_user<false, false, kNodesQuantized>,
+         k_trace_user<false, false, kNodesWalk>},
+        {k_trace_user<true, false, kNodesFull>, k_trace_user<true, false, kNodesQuantized>,
+         k_trace_user<true, false, kNodesWalk>}};
+    const Kernel k = count ? (any ? k_trace_user<true, true, kNodesFull> : k_trace_user<false, true, kNodesFull>)
+                           : walks[any][walk_format(sc->ds)];
     int per_sm = 1;
     AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 128, 0));
     size_t need = (n + 127) / 128;
