@@ -248,6 +248,33 @@ __device__ __forceinline__ int32_t push_ordered(Children c, int32_t* stack, int&
     return sp > 0 ? stack[--sp] : kTraversalDone;
 }
 
+// Turns the hit children's entry distances into keys that sort the one
+// entered last to the front (misses stay behind).
+__device__ __forceinline__ void farthest_first(Children& c) {
+    c.t0 = c.t0 == INFINITY ? INFINITY : -c.t0;
+    c.t1 = c.t1 == INFINITY ? INFINITY : -c.t1;
+    c.t2 = c.t2 == INFINITY ? INFINITY : -c.t2;
+    c.t3 = c.t3 == INFINITY ? INFINITY : -c.t3;
+}
+
+// Order for occlusion: descend into the child entered last, push the other
+// hit children as three of the comparators leave them. The answer does not
+// depend on the order, and near the origin a ray mostly passes by what it
+// left; the far children hold its occluder sooner (visits per ray, random
+// segments: interior 11.4 nearest first, 8.5 farthest first; sphere field
+// 10.0 and 3.7; rays to the lights 17.9 and 18.1, 16.7 and 15.5).
+__device__ __forceinline__ int32_t push_occlusion(Children c, int32_t* stack, int& sp) {
+    farthest_first(c);
+    order2(c.t0, c.c0, c.t1, c.c1);
+    order2(c.t2, c.c2, c.t3, c.c3);
+    order2(c.t0, c.c0, c.t2, c.c2);
+    if (c.t3 != INFINITY) stack[sp++] = c.c3;
+    if (c.t2 != INFINITY) stack[sp++] = c.c2;
+    if (c.t1 != INFINITY) stack[sp++] = c.c1;
+    if (c.t0 != INFINITY) return c.c0;
+    return sp > 0 ? stack[--sp] : kTraversalDone;
+}
+
 // Visits node `node` in the scene's own format, nearest child first (the
 // canonical walk, whose work is counted).
 __device__ __forceinline__ int32_t visit_node(const DevScene& S, int32_t node, const RayPre& rp, float tfar,
@@ -423,6 +450,18 @@ __device__ __forceinline__ TraceResult traverse_fast(const DevScene& S, v3 o, v3
 //   done(tag, r): called once per ray, by the lanes finishing in the same
 //                 round together (warp collectives inside are allowed).
 constexpr int kRefillLanes = 16;
+// Over walk nodes, a round leaves the inner nodes once fewer than this many
+// of the lanes still walking hold no leaf; waiting for the last of them left
+// 17 of 32 lanes active per visit on the interior and 15 on its occlusion
+// rays, 6 leaves 22 and 21. (4, 8 and 12 were slower there; over the
+// full-precision nodes of small trees, where rays are short, waiting for the
+// last lane stays the faster by 0.5%.)
+constexpr int kWalkLanes = 6;
+// Resident 128-thread blocks per SM the traversal kernels are compiled for:
+// 9 keep them within 56 registers. Against 8 (64 registers) and 10 (48): Cornell
+// GGX 1024^2 at 64 spp 37.8 / 38.6 / 38.9 ms, interior 1080p at 8 spp 40.3 /
+// 41.2 / 42.1 ms, 2.07M interior rays 475 / 486 / 512 us.
+constexpr int kTraceBlocks = 9;
 
 // Kinds of queue: closest hits, any hits, or both mixed (the load callback
 // then sets `any` per ray: load(i, o, d, tmin, tmax, any)).
@@ -473,12 +512,23 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
         if (!have) continue;
         // One round of traverse_fast.
         while (node >= 0) {
-            node = push_ordered(load_children<NODES>(S, node, rp, r.t), stack, sp);
+            Children c = load_children<NODES>(S, node, rp, r.t);
+            if constexpr (KIND == kQueueAny && NODES == kNodesWalk) {
+                node = push_occlusion(c, stack, sp);
+            } else {
+                if constexpr (KIND == kQueueMixed && NODES == kNodesWalk)
+                    if (any) farthest_first(c);
+                node = push_ordered(c, stack, sp);
+            }
             if (node < 0 && node != kTraversalDone && leaf == 0) {
                 leaf = node;
                 node = sp > 0 ? stack[--sp] : kTraversalDone;
             }
-            if (!__any_sync(__activemask(), leaf == 0)) break;
+            if constexpr (NODES == kNodesWalk) {
+                if (__popc(__ballot_sync(__activemask(), leaf == 0)) < kWalkLanes) break;
+            } else {
+                if (!__any_sync(__activemask(), leaf == 0)) break;
+            }
         }
         while (leaf < 0) {
             int32_t code = ~leaf;

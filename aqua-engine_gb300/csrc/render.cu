@@ -226,7 +226,7 @@ __device__ __forceinline__ void ltrain_add(float4* L, uint32_t id, v3 c) {
 }
 
 template <bool SORTED, bool COUNT, int NODES>
-__global__ void __launch_bounds__(128) k_trace_ext(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
+__global__ void __launch_bounds__(128, kTraceBlocks) k_trace_ext(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
                                                    uint32_t cnt_out) {
     grid_dep_wait();
     grid_dep_launch();
@@ -592,7 +592,7 @@ __device__ __forceinline__ void shadow_done(const WaveParams& P, const WavePtrs&
 }
 
 template <bool COUNT, bool NRC, int NODES>
-__global__ void __launch_bounds__(128) k_shadow(DevScene S, WaveParams P, WavePtrs W) {
+__global__ void __launch_bounds__(128, kTraceBlocks) k_shadow(DevScene S, WaveParams P, WavePtrs W) {
     grid_dep_wait();
     grid_dep_launch();
     uint32_t n = W.counters[kCntShadow];
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(128) k_shadow(DevScene S, WaveParams P, WavePt
 // slot's shadow contribution of bounce k lands before bounce k + 1 is
 // shaded, as in the three-launch pipeline.
 template <bool NRC, int NODES>
-__global__ void __launch_bounds__(128) k_trace_fused(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
+__global__ void __launch_bounds__(128, kTraceBlocks) k_trace_fused(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
                                                      uint32_t cnt_out, uint32_t sh_in, uint32_t sh_out) {
     grid_dep_wait();
     grid_dep_launch();

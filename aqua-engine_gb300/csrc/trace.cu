@@ -9,7 +9,7 @@
 namespace aq {
 
 template <bool ANY, bool COUNT, int NODES>
-__global__ void __launch_bounds__(128) k_trace_user(DevScene S, const float4* __restrict__ rays, size_t n,
+__global__ void __launch_bounds__(128, kTraceBlocks) k_trace_user(DevScene S, const float4* __restrict__ rays, size_t n,
                                                     float4* __restrict__ hits, unsigned long long* stats) {
     uint32_t nodes = 0, tris = 0;
     auto store = [&](size_t i, const TraceResult& r) {
