@@ -467,9 +467,9 @@ constexpr int kTraceBlocks = 9;
 // then sets `any` per ray: load(i, o, d, tmin, tmax, any)).
 enum { kQueueClosest = 0, kQueueAny = 1, kQueueMixed = 2 };
 
-template <int KIND, int NODES, class Load, class Done>
-__device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, uint32_t* cursor, Load load,
-                                               Done done) {
+template <int KIND, int NODES, bool SPARSE, class Load, class Done>
+__device__ __forceinline__ void traverse_lanes(const DevScene& S, uint32_t n, uint32_t width, uint32_t* cursor,
+                                               Load load, Done done) {
     const unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     RayPre rp;
@@ -480,39 +480,40 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
     int32_t node = kTraversalDone, leaf = 0;
     uint32_t tag = 0;
     bool have = false, drained = false, any = KIND == kQueueAny;
-    // A queue shorter than the grid's lanes is spread over all its warps, few
-    // lanes each: a warp then takes as long as the longest of its few rays, not
-    // as the union of 32 divergent ones, and more warps hide each other's
-    // fetches (a cached 1080p frame, whose last ten iterations trace 10-40k
-    // rays: 3.39 -> 3.24 ms; a 64 x 64 thumbnail 0.57 -> 0.42 ms).
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const int width = (int)min(32u, (n + warps - 1u) / warps);
-    if (width == 0) return;
+    auto take = [&](uint32_t i) {
+        v3 o, d;
+        float tmin, tmax;
+        if constexpr (KIND == kQueueMixed) tag = load(i, o, d, tmin, tmax, any);
+        else tag = load(i, o, d, tmin, tmax);
+        rp.o = o;
+        rp.invd = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+        rp.tmin = tmin;
+        rp.tmax = tmax;
+        sh = make_shear(o, d);
+        r.t = tmax; r.u = 0.0f; r.v = 0.0f; r.tri = -1; r.id = 0x7fffffff;
+        sp = 0;
+        node = 0;
+        leaf = 0;
+        have = true;
+    };
+    if constexpr (SPARSE) {
+        // The warp's share, dealt without the counter: thousands of warps
+        // asking one address take microseconds.
+        const uint32_t i = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * width + (uint32_t)lane;
+        if ((uint32_t)lane < width && i < n) take(i);
+    }
     while (true) {
-        const unsigned idle = __ballot_sync(kFull, !have && lane < width);
-        if (!drained && __popc(idle) >= min(kRefillLanes, width)) {
-            const int leader = __ffs(idle) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (base + (uint32_t)__popc(idle) >= n) drained = true;
-            if (!have && lane < width) {
-                const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (i < n) {
-                    v3 o, d;
-                    float tmin, tmax;
-                    if constexpr (KIND == kQueueMixed) tag = load(i, o, d, tmin, tmax, any);
-                    else tag = load(i, o, d, tmin, tmax);
-                    rp.o = o;
-                    rp.invd = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-                    rp.tmin = tmin;
-                    rp.tmax = tmax;
-                    sh = make_shear(o, d);
-                    r.t = tmax; r.u = 0.0f; r.v = 0.0f; r.tri = -1; r.id = 0x7fffffff;
-                    sp = 0;
-                    node = 0;
-                    leaf = 0;
-                    have = true;
+        if constexpr (!SPARSE) {
+            const unsigned idle = __ballot_sync(kFull, !have);
+            if (!drained && __popc(idle) >= kRefillLanes) {
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if (lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(idle));
+                base = __shfl_sync(kFull, base, leader);
+                if (base + (uint32_t)__popc(idle) >= n) drained = true;
+                if (!have) {
+                    const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+                    if (i < n) take(i);
                 }
             }
         }
@@ -532,8 +533,8 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
                 leaf = node;
                 node = sp > 0 ? stack[--sp] : kTraversalDone;
             }
-            if constexpr (NODES == kNodesWalk) {
-                if (__popc(__ballot_sync(__activemask(), leaf == 0)) < (width == 32 ? kWalkLanes : 1)) break;
+            if constexpr (NODES == kNodesWalk && !SPARSE) {
+                if (__popc(__ballot_sync(__activemask(), leaf == 0)) < kWalkLanes) break;
             } else {
                 if (!__any_sync(__activemask(), leaf == 0)) break;
             }
@@ -575,6 +576,22 @@ __device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, ui
             have = false;
         }
     }
+}
+
+// A queue shorter than the grid's lanes is spread over all its warps, few
+// lanes each: a warp then takes as long as the longest of its few rays, not as
+// the union of 32 divergent ones, and more warps hide each other's fetches (a
+// cached 1080p frame, whose last ten iterations trace 10-40k rays: 3.39 -> 3.24
+// ms; a 64 x 64 thumbnail 0.57 -> 0.41 ms). Two copies of the loop, because one
+// with a variable width spills registers on full queues (Cornell GGX 1024^2
+// 155.1 -> 157.4 ms).
+template <int KIND, int NODES, class Load, class Done>
+__device__ __forceinline__ void traverse_queue(const DevScene& S, uint32_t n, uint32_t* cursor, Load load,
+                                               Done done) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t width = (n + warps - 1u) / warps;
+    if (width < 32u) traverse_lanes<KIND, NODES, true>(S, n, width, cursor, load, done);
+    else traverse_lanes<KIND, NODES, false>(S, n, 32u, cursor, load, done);
 }
 
 // Warp-aggregated append: lanes with pred set get consecutive slots of *ctr.

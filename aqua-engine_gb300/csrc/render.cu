@@ -186,6 +186,15 @@ __device__ __forceinline__ uint32_t block_append(uint32_t* ctr, bool pred, uint3
     return k;
 }
 
+// *sum += a * b, one rounding per channel: spelled out, so that every variant
+// of the shading kernel rounds alike (the compiler may fuse a product into
+// the addition in one variant and not in another).
+__device__ __forceinline__ void add_product(float4* sum, v3 a, v3 b) {
+    float4 f = *sum;
+    f.x = fmaf(a.x, b.x, f.x); f.y = fmaf(a.y, b.y, f.y); f.z = fmaf(a.z, b.z, f.z);
+    *sum = f;
+}
+
 __device__ __forceinline__ void film_add(float4* film, uint32_t pixel, v3 c) {
     float4 f = film[pixel];
     f.x += c.x; f.y += c.y; f.z += c.z;
@@ -305,10 +314,7 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
                                                uint32_t cnt_out, uint32_t cnt_sh) {
     __shared__ float lut[256];
     __shared__ uint32_t prefix[257];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        float c = (float)i / 255.0f;
-        lut[i] = c <= 0.04045f ? c / 12.92f : powf((c + 0.055f) / 1.055f, 2.4f);
-    }
+    if (S.n_texs > 0) fill_srgb_lut(lut);
     grid_dep_wait();
     grid_dep_launch();
     if (blockIdx.x == 0 && threadIdx.x == 0) W.counters[kCntFetchTrace] = 0;  // for the next traversal launch
@@ -370,8 +376,8 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
         if (tri < 0) {
             v3 e = mk(S.env[0], S.env[1], S.env[2]);
             if (e.x > 0.0f || e.y > 0.0f || e.z > 0.0f) {
-                if (!NRC || (int)depth <= P.max_depth) film_add(W.film, pixel, thr * e);
-                if (NRC && tag) ltrain_add(W.ltrain, train_id, thr * e);
+                if (!NRC || (int)depth <= P.max_depth) add_product(W.film + pixel, thr, e);
+                if (NRC && tag) add_product(W.ltrain + train_id, thr, e);
             }
         } else {
             float4 rd = W.ray_d[s];
@@ -396,9 +402,10 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
                     }
                     // Past max_depth a training path gathers for its targets only:
                     // the image keeps the plain estimator's depth.
+                    const v3 tl = thr * f3(L.le), w3 = mk(w, w, w);
                     if (!(NRC && P.visualize) && (!NRC || (int)depth <= P.max_depth))
-                        film_add(W.film, pixel, thr * f3(L.le) * w);
-                    if (NRC && tag) ltrain_add(W.ltrain, train_id, thr * f3(L.le) * w);
+                        add_product(W.film + pixel, tl, w3);
+                    if (NRC && tag) add_product(W.ltrain + train_id, tl, w3);
                 }
             }
             // Training paths run train_span bounces past the last vertex
@@ -758,14 +765,20 @@ using TraceKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t)
 using ShadowKernel = void (*)(DevScene, WaveParams, WavePtrs);
 using FusedKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t, uint32_t, uint32_t);
 
-static TraceKernel trace_kernel(const DevScene& S, bool sorted, bool count) {
+// The first iteration's rays are the camera's: neighbours walk the same nodes,
+// which the full-precision ones serve from L1 to the whole warp, so they are
+// walked there whatever the later, incoherent rays use (2.07M camera rays of
+// the interior: 377 us against 430 us over its walk nodes).
+static int first_format(const DevScene& S) { return S.qbvh ? kNodesQuantized : kNodesFull; }
+
+static TraceKernel trace_kernel(int format, bool sorted, bool count) {
     static constexpr TraceKernel walks[2][3] = {
         {k_trace_ext<false, false, kNodesFull>, k_trace_ext<false, false, kNodesQuantized>,
          k_trace_ext<false, false, kNodesWalk>},
         {k_trace_ext<true, false, kNodesFull>, k_trace_ext<true, false, kNodesQuantized>,
          k_trace_ext<true, false, kNodesWalk>}};
     if (count) return sorted ? k_trace_ext<true, true, kNodesFull> : k_trace_ext<false, true, kNodesFull>;
-    return walks[sorted][walk_format(S)];
+    return walks[sorted][format];
 }
 
 static ShadowKernel shadow_kernel(const DevScene& S, bool count, bool nrc) {
@@ -776,10 +789,10 @@ static ShadowKernel shadow_kernel(const DevScene& S, bool count, bool nrc) {
     return count ? k_shadow<true, false, kNodesFull> : walks[nrc][walk_format(S)];
 }
 
-static FusedKernel fused_kernel(const DevScene& S) {
+static FusedKernel fused_kernel(int format) {
     static constexpr FusedKernel walks[3] = {k_trace_fused<true, kNodesFull>, k_trace_fused<true, kNodesQuantized>,
                                              k_trace_fused<true, kNodesWalk>};
-    return walks[walk_format(S)];
+    return walks[format];
 }
 
 template <class K>
@@ -863,6 +876,21 @@ SlotPlan plan_slots(size_t pixels, int spp, const aqua_tuning& tune, bool deep) 
 }
 }  // namespace
 
+// Most iterations a wavefront needs: a slot runs its work items one after
+// another, and an item is over at the latest when its vertex at the depth limit
+// is shaded.
+static uint64_t iteration_bound(size_t pixels, const SlotPlan& plan, int spp, int depth_limit) {
+    const uint64_t items = plan.replicas > 1 ? ((uint64_t)spp + plan.replicas - 1) / plan.replicas
+                                             : (uint64_t)((pixels + plan.slots - 1) / plan.slots) * (uint64_t)spp;
+    return items * (uint64_t)(depth_limit + 1);
+}
+
+// Every path must have ended within the iteration bound.
+static void check_drained(uint64_t paths, size_t pixels, int spp) {
+    if (paths != (uint64_t)pixels * (uint64_t)spp)
+        throw Error(AQUA_ERR_TIMEOUT, "wavefront did not drain within the iteration bound");
+}
+
 // Rows of the camera image a render covers (aqua_integrator_cfg row subset);
 // sets the parameters' row fields and returns the film's pixel count.
 static size_t plan_rows(const aqua_integrator_cfg& cfg, const DevCamera& cam, WaveParams& P) {
@@ -920,7 +948,8 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     if (bt != 128 && bt != 64 && bt != 32) throw Error(AQUA_ERR_INVALID_ARG, "block_trace must be 32, 64 or 128");
     if (bs != 128 && bs != 64 && bs != 32) throw Error(AQUA_ERR_INVALID_ARG, "block_shade must be 32, 64 or 128");
 
-    const TraceKernel trace_k = trace_kernel(S, sorted, count);
+    const TraceKernel trace_k = trace_kernel(walk_format(S), sorted, count);
+    const TraceKernel first_k = trace_kernel(first_format(S), sorted, count);
     const bool full = S.mext != nullptr;  // some material sets the full model's lobes
     auto shade_k = full ? (sorted ? k_shade<true, false, true> : k_shade<false, false, true>)
                         : (sorted ? k_shade<true> : k_shade<false>);
@@ -948,15 +977,20 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
         AQ_CUDA(cudaGetLastError());
         ++launches;
     }
+    // Iterations go out in chunks; the queue length after each comes back
+    // while the next one runs. A render whose bound lies within the first
+    // chunk (one sample per slot) launches exactly that many and asks
+    // nothing; otherwise the chunks shrink once slots begin to run out of
+    // work, so that few empty iterations follow the last path.
     const int chunk = tune.iters_per_graph > 0 ? tune.iters_per_graph : 16;
+    const uint64_t bound = iteration_bound(pixels, plan, cfg.spp, cfg.max_depth);
     uint64_t iter = 0;
     unsigned int* pc = ctx->pinned_counter;
     cudaEvent_t chunk_ev[2] = {tt.get(), tt.get()};
-    int c = 0;
-    const uint64_t max_iters = (uint64_t)(cfg.max_depth + 2) * (uint64_t)cfg.spp *
-                                   ((pixels + slots - 1) / slots) + 64;
-    while (true) {
-        for (int k = 0; k < chunk; ++k, ++iter) {
+    uint64_t step = (uint64_t)chunk;
+    for (int c = 0; iter < bound; ++c) {
+        const uint64_t end = std::min(bound, iter + step);
+        for (; iter < end; ++iter) {
             uint32_t in = (uint32_t)(iter & 1), out = 1u - in;
             W.q_in = w.q[in];
             W.q_out = w.q[out];
@@ -964,7 +998,7 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
             // the events barely perturb the launch stream.
             bool timed = timing && (iter % kStageTimingStride) == 0;
             if (timed) tt.begin();
-            launch_chained(trace_k, g_trace, bt, 0, st, S, P, W, in, out);
+            launch_chained(iter == 0 ? first_k : trace_k, g_trace, bt, 0, st, S, P, W, in, out);
             if (timed) { tt.end(); ts.begin(); }
             launch_chained(shade_k, g_shade, bs, 0, st, S, P, W, in, out, (uint32_t)kCntShadow);
             if (timed) { ts.end(); tsh.begin(); }
@@ -973,18 +1007,13 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
             launches += 3;
         }
         AQ_CUDA(cudaGetLastError());
+        if (iter >= bound) break;
         AQ_CUDA(cudaMemcpyAsync(&pc[c & 1], &w.counters[iter & 1], 4, cudaMemcpyDeviceToHost, st));
         AQ_CUDA(cudaEventRecord(chunk_ev[c & 1], st));
         if (c > 0) {
             AQ_CUDA(cudaEventSynchronize(chunk_ev[(c - 1) & 1]));
             if (pc[(c - 1) & 1] == 0) break;
-        }
-        ++c;
-        if (iter > max_iters) {
-            AQ_CUDA(cudaStreamSynchronize(st));
-            if (pc[(c - 1) & 1] != 0)
-                throw Error(AQUA_ERR_TIMEOUT, "wavefront did not drain within the iteration bound");
-            break;
+            if (pc[(c - 1) & 1] < slots) step = std::min<uint64_t>(step, 4);
         }
     }
     float* dst = (flags & AQUA_RENDER_DEVICE_FILM) ? rgb_out : w.out_rgb;
@@ -1004,6 +1033,7 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     unsigned long long hs[16];
     AQ_CUDA(cudaMemcpyAsync(hs, w.stats, 8 * 16, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
+    check_drained(hs[kStatPaths], pixels, cfg.spp);
     if (stats) {
         memset(stats, 0, sizeof(*stats));
         float ms = 0.0f;
@@ -1203,7 +1233,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     W.q_pix = nw.q_pix; W.q_raw = nw.q_raw; W.rec = nw.rec; W.ltrain = nw.ltrain; W.lsnap = nw.lsnap;
     W.spread = nw.spread;
 
-    const TraceKernel trace_k = trace_kernel(S, sorted, false);
+    const TraceKernel trace_k = trace_kernel(walk_format(S), sorted, false);
     auto shade_k = S.mext ? (sorted ? k_shade<true, true, true> : k_shade<false, true, true>)
                           : (sorted ? k_shade<true, true> : k_shade<false, true>);
     const ShadowKernel shadow_k = shadow_kernel(S, false, true);
@@ -1218,7 +1248,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     // the 1080p interior). Deep plain renders stay on three launches, where
     // the fused launch measured 2.3% slower (Cornell GGX 1024^2).
     const bool fused = !sorted;
-    const FusedKernel fused_k = fused_kernel(S);
+    const FusedKernel fused_k = fused_kernel(walk_format(S)), first_k = fused_kernel(first_format(S));
     int g_fused = fused ? grid_for(ctx, fused_k, 128, tune.blocks_per_sm) : 0;
 
     cudaEvent_t ev[4];
@@ -1238,21 +1268,20 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
         AQ_CUDA(cudaGetLastError());
         ++launches;
     }
-    // A 1-spp frame drains within train_depth + 1 iterations: no empty
-    // iterations before the host's check.
-    const int chunk = std::min(tune.iters_per_graph > 0 ? tune.iters_per_graph : 16, train_depth + 2);
-    const uint64_t max_iters =
-        (uint64_t)(train_depth + 2) * (uint64_t)cfg.spp * ((pixels + slots - 1) / slots) + 64;
+    // A 1-spp frame is done after train_depth + 1 iterations, all in one chunk.
+    const uint64_t bound = iteration_bound(pixels, plan, cfg.spp, std::max(train_depth, cfg.max_depth));
+    const uint64_t chunk = (uint64_t)std::min(tune.iters_per_graph > 0 ? tune.iters_per_graph : 16, train_depth + 1);
     uint64_t iter = 0;
     unsigned int* pc = ctx->pinned_counter;
     while (true) {
-        for (int k = 0; k < chunk; ++k, ++iter) {
+        const uint64_t end = std::min(bound, iter + chunk);
+        for (; iter < end; ++iter) {
             uint32_t in = (uint32_t)(iter & 1), out = 1u - in;
             W.q_in = w.q[in];
             W.q_out = w.q[out];
             if (fused) {
                 const uint32_t sh_now = in ? kCntShadow1 : kCntShadow, sh_prev = in ? kCntShadow : kCntShadow1;
-                launch_chained(fused_k, g_fused, 128, 0, st, S, P, W, in, out, sh_prev, sh_now);
+                launch_chained(iter == 0 ? first_k : fused_k, g_fused, 128, 0, st, S, P, W, in, out, sh_prev, sh_now);
                 launch_chained(shade_k, g_shade, 128, 0, st, S, P, W, in, out, sh_now);
                 launches += 2;
                 continue;
@@ -1266,8 +1295,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
         AQ_CUDA(cudaMemcpyAsync(&pc[8], &w.counters[iter & 1], 4, cudaMemcpyDeviceToHost, st));
         AQ_CUDA(cudaMemcpyAsync(&pc[9], &w.counters[kCntQuery], 12, cudaMemcpyDeviceToHost, st));
         AQ_CUDA(cudaStreamSynchronize(st));
-        if (pc[8] == 0) break;
-        if (iter > max_iters) throw Error(AQUA_ERR_TIMEOUT, "wavefront did not drain within the iteration bound");
+        if (pc[8] == 0 || iter >= bound) break;
     }
     if (fused) {  // the shadow rays of the last shading launch
         const uint32_t in = (uint32_t)(iter & 1), out = 1u - in;
@@ -1335,6 +1363,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     unsigned long long hs[16];
     AQ_CUDA(cudaMemcpyAsync(hs, w.stats, 8 * 16, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
+    check_drained(hs[kStatPaths], pixels, cfg.spp);
     nrc_check_tc(ctx, net);
     if (stats) {
         memset(stats, 0, sizeof(*stats));
@@ -1463,7 +1492,7 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
     AQ_CUDA(cudaMemsetAsync(W.counters, 0, 4 * kNoAllocCounters, st));
     AQ_CUDA(cudaMemsetAsync(W.stats, 0, 8 * kNoAllocStats, st));
 
-    const TraceKernel trace_k = trace_kernel(S, false, false);
+    const TraceKernel trace_k = trace_kernel(walk_format(S), false, false);
     auto shade_k = S.mext ? k_shade<false, false, true> : k_shade<false>;
     const ShadowKernel shadow_k = shadow_kernel(S, false, false);
     int g_trace = grid_for(ctx, trace_k, 128, 0);
@@ -1478,13 +1507,12 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
         AQ_CUDA(cudaGetLastError());
         ++launches;
     }
-    const int chunk = 16;
-    const uint64_t max_iters =
-        (uint64_t)(cfg.max_depth + 2) * (uint64_t)cfg.spp * ((pixels + slots - 1) / slots) + 64;
-    uint64_t iter = 0;
+    const uint64_t bound = iteration_bound(pixels, SlotPlan{slots, 1}, cfg.spp, cfg.max_depth);
+    uint64_t iter = 0, step = 16;
     unsigned int* pc = ctx->pinned_counter;  // pinned when the context was created
-    while (true) {
-        for (int k = 0; k < chunk; ++k, ++iter) {
+    while (iter < bound) {
+        const uint64_t end = std::min(bound, iter + step);
+        for (; iter < end; ++iter) {
             uint32_t in = (uint32_t)(iter & 1), out = 1u - in;
             W.q_in = q[in];
             W.q_out = q[out];
@@ -1494,10 +1522,10 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
             launches += 3;
         }
         AQ_CUDA(cudaGetLastError());
+        if (iter >= bound) break;
         AQ_CUDA(cudaMemcpyAsync(&pc[4], &W.counters[iter & 1], 4, cudaMemcpyDeviceToHost, st));
         AQ_CUDA(cudaStreamSynchronize(st));
         if (pc[4] == 0) break;
-        if (iter > max_iters) throw Error(AQUA_ERR_TIMEOUT, "wavefront did not drain within the iteration bound");
     }
     {
         int g = (int)std::min<size_t>((pixels + 255) / 256, (size_t)ctx->num_sms * 16);
@@ -1508,6 +1536,7 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
     unsigned long long hs[kNoAllocStats];
     AQ_CUDA(cudaMemcpyAsync(hs, W.stats, sizeof(hs), cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
+    check_drained(hs[kStatPaths], pixels, cfg.spp);
     if (stats) {
         memset(stats, 0, sizeof(*stats));
         stats->paths = hs[kStatPaths];

@@ -8,47 +8,49 @@
 
 namespace aq {
 
-template <bool ANY, bool COUNT, int NODES>
-__global__ void __launch_bounds__(128, kTraceBlocks) k_trace_user(DevScene S, const float4* __restrict__ rays, size_t n,
-                                                    float4* __restrict__ hits, unsigned long long* stats) {
+template <bool ANY>
+__device__ __forceinline__ void store_hit(float4* hits, size_t i, const TraceResult& r) {
+    float4 h;
+    if (ANY) h = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(r.tri >= 0 ? 1 : -1));
+    else if (r.tri < 0) h = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+    else h = make_float4(r.t, r.u, r.v, __int_as_float(r.id));
+    hits[i] = h;
+}
+
+// The renderer's traversal over the caller's rays.
+template <bool ANY, int NODES>
+__global__ void __launch_bounds__(128, kTraceBlocks) k_trace_user(DevScene S, const float4* __restrict__ rays,
+                                                                  uint32_t n, float4* __restrict__ hits,
+                                                                  uint32_t* cursor) {
+    traverse_queue<ANY ? kQueueAny : kQueueClosest, NODES>(
+        S, n, cursor,
+        [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
+            float4 a = ldg_(rays + 2 * (size_t)i), b = ldg_(rays + 2 * (size_t)i + 1);
+            o = mk(a.x, a.y, a.z);
+            d = mk(b.x, b.y, b.z);
+            tmin = a.w;
+            tmax = b.w;
+            return i;
+        },
+        [&](uint32_t i, const TraceResult& r) { store_hit<ANY>(hits, i, r); });
+}
+
+// The canonical walk, counted: stats[0] += node visits, stats[1] += triangle tests.
+template <bool ANY>
+__global__ void __launch_bounds__(128) k_trace_count(DevScene S, const float4* __restrict__ rays, size_t n,
+                                                     float4* __restrict__ hits, unsigned long long* stats) {
     uint32_t nodes = 0, tris = 0;
-    auto store = [&](size_t i, const TraceResult& r) {
-        float4 h;
-        if (ANY) h = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(r.tri >= 0 ? 1 : -1));
-        else if (r.tri < 0) h = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
-        else h = make_float4(r.t, r.u, r.v, __int_as_float(r.id));
-        hits[i] = h;
-    };
-    if (!COUNT && n < (1ull << 31)) {
-        // The renderer's traversal: persistent lanes with ray replacement;
-        // stats[2] is the queue cursor.
-        traverse_queue<ANY ? kQueueAny : kQueueClosest, NODES>(
-            S, (uint32_t)n, reinterpret_cast<uint32_t*>(stats + 2),
-            [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
-                float4 a = ldg_(rays + 2 * (size_t)i), b = ldg_(rays + 2 * (size_t)i + 1);
-                o = mk(a.x, a.y, a.z);
-                d = mk(b.x, b.y, b.z);
-                tmin = a.w;
-                tmax = b.w;
-                return i;
-            },
-            store);
-        return;
-    }
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float4 a = ldg_(rays + 2 * i), b = ldg_(rays + 2 * i + 1);
-        store(i, COUNT ? traverse<ANY, true>(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, nodes, tris)
-                       : traverse_fast<kNodesOwn>(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, ANY));
+        store_hit<ANY>(hits, i, traverse<ANY, true>(S, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, nodes, tris));
     }
-    if (COUNT) {
-        for (int o = 16; o > 0; o >>= 1) {
-            nodes += __shfl_down_sync(0xffffffffu, nodes, o);
-            tris += __shfl_down_sync(0xffffffffu, tris, o);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&stats[0], (unsigned long long)nodes);
-            atomicAdd(&stats[1], (unsigned long long)tris);
-        }
+    for (int o = 16; o > 0; o >>= 1) {
+        nodes += __shfl_down_sync(0xffffffffu, nodes, o);
+        tris += __shfl_down_sync(0xffffffffu, tris, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&stats[0], (unsigned long long)nodes);
+        atomicAdd(&stats[1], (unsigned long long)tris);
     }
 }
 
@@ -129,22 +131,31 @@ void trace_rays(aqua_ctx* ctx, aqua_scene* sc, const aqua_ray* rays, size_t n, a
     if (!ctx->trace_stats.ptr) dev_alloc(ctx, ctx->trace_stats, 64);
     unsigned long long* d_stats = (unsigned long long*)ctx->trace_stats.ptr;
     AQ_CUDA(cudaMemsetAsync(d_stats, 0, 24, st));  // node and triangle counters, queue cursor
-    using Kernel = void (*)(DevScene, const float4*, size_t, float4*, unsigned long long*);
-    static constexpr Kernel walks[2][3] = {  // by any, walk_format
-        {k_trace_user<false, false, kNodesFull>, k_trace_user<false, false, kNodesQuantized>,
-         k_trace_user<false, false, kNodesWalk>},
-        {k_trace_user<true, false, kNodesFull>, k_trace_user<true, false, kNodesQuantized>,
-         k_trace_user<true, false, kNodesWalk>}};
-    const Kernel k = count ? (any ? k_trace_user<true, true, kNodesFull> : k_trace_user<false, true, kNodesFull>)
-                           : walks[any][walk_format(sc->ds)];
+    using Walk = void (*)(DevScene, const float4*, uint32_t, float4*, uint32_t*);
+    static constexpr Walk walks[2][3] = {  // by any, walk_format
+        {k_trace_user<false, kNodesFull>, k_trace_user<false, kNodesQuantized>, k_trace_user<false, kNodesWalk>},
+        {k_trace_user<true, kNodesFull>, k_trace_user<true, kNodesQuantized>, k_trace_user<true, kNodesWalk>}};
+    const Walk walk = walks[any][walk_format(sc->ds)];
+    const auto counted = any ? k_trace_count<true> : k_trace_count<false>;
     int per_sm = 1;
-    AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 128, 0));
-    size_t need = (n + 127) / 128;
+    if (count) AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, counted, 128, 0));
+    else AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk, 128, 0));
+    // A short queue is dealt to all warps (traverse_queue): down to one ray each.
+    const size_t need = count ? (n + 127) / 128 : (n + 3) / 4;
     int grid = (int)std::min<size_t>(need, (size_t)ctx->num_sms * (size_t)std::max(per_sm, 1));
     EventPair ev;
     AQ_CUDA(cudaEventRecord(ev.e[0], st));
-    k<<<grid, 128, 0, st>>>(sc->ds, d_rays, n, d_hits, d_stats);
-    AQ_CUDA(cudaGetLastError());
+    if (count) {
+        counted<<<grid, 128, 0, st>>>(sc->ds, d_rays, n, d_hits, d_stats);
+        AQ_CUDA(cudaGetLastError());
+    }
+    constexpr size_t kChunk = (size_t)1 << 30;  // rays per launch: the queue counts in 32 bits
+    for (size_t i = 0; !count && i < n; i += kChunk) {
+        if (i > 0) AQ_CUDA(cudaMemsetAsync(d_stats + 2, 0, 8, st));
+        walk<<<grid, 128, 0, st>>>(sc->ds, d_rays + 2 * i, (uint32_t)std::min(kChunk, n - i), d_hits + i,
+                                   reinterpret_cast<uint32_t*>(d_stats + 2));
+        AQ_CUDA(cudaGetLastError());
+    }
     AQ_CUDA(cudaEventRecord(ev.e[1], st));
     if (!dev) AQ_CUDA(cudaMemcpyAsync(out, d_hits, 16 * n, cudaMemcpyDeviceToHost, st));
     unsigned long long hs[2] = {0, 0};
