@@ -127,8 +127,7 @@ struct NrcNet {
     float* ema = nullptr;    // exponential moving average of w (inference weights)
     uint2* frag_inf = nullptr;  // forward fragments of the inference weights
     uint8_t* img_tc = nullptr;  // inference weights in the tcgen05 shared-memory layout
-    uint8_t* img_tc_w = nullptr;  // the trained weights w in that layout (training forward)
-    uint8_t* img_tc_bwd = nullptr;  // W6^T, W5^T..W2^T of w in that layout (backward)
+    uint8_t* img_tc_w = nullptr;  // the trained weights w in that layout (training)
     uint32_t* tc_err = nullptr; // set by the tcgen05 kernel when a wait expired
     int forward_tc = 0;         // 1: inference runs on tcgen05 (else mma.sync)
     float ema_decay = 0.0f;  // 0 = inference uses w itself
@@ -138,7 +137,8 @@ struct NrcNet {
     uint32_t* acts = nullptr;  // H1..H5 bf16 (5 x rows x 64)
     uint32_t* deltas = nullptr;// delta1..delta5 bf16 (5 x rows x 64)
     uint32_t* d6 = nullptr;    // dY bf16 (rows x 16)
-    float* partial = nullptr;  // per-chunk weight gradients
+    float* partial = nullptr;  // partial weight gradients (per CTA, or per chunk of rows)
+    double* losses = nullptr;  // partial loss sums (tcgen05)
     int64_t step = 0;
     float lr = 1e-2f, beta1 = 0.9f, beta2 = 0.99f, eps = 1e-8f;
     float bmin[3] = {0, 0, 0}, bext[3] = {1, 1, 1};
@@ -232,8 +232,7 @@ struct aqua_ctx {
     aq::DevBuf trace_rays, trace_hits;       // staging for host-pointer traces
     aq::DevBuf persist_film;                 // device film of host-film persistent renders
     bool nrc_tc_ready = false;               // tcgen05 inference kernel configured on this device
-    bool nrc_tc_bwd_ready = false;           // and the tcgen05 backward kernel
-    bool nrc_tc_wg_ready = false;            // and the tcgen05 weight-gradient kernel
+    bool nrc_tc_train_ready = false;         // and the tcgen05 training kernel
     aq::DevBuf trace_stats;
 };
 
@@ -300,17 +299,14 @@ void nrc_train_step_dev(aqua_ctx* ctx, NrcNet& net, const uint16_t* X, const flo
 void nrc_encode_dev(aqua_ctx* ctx, NrcNet& net, const float* raw, int n, uint16_t* X);
 // tcgen05 inference (nrc_tc.cu)
 size_t nrc_tc_weight_bytes();
-// All three tcgen05 weight images: forward of w and of inf, backward of w.
-void nrc_pack_tc(aqua_ctx* ctx, const float* w, const float* inf, void* img_w, void* img_inf, void* img_bwd);
-void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n, float* out, uint32_t* err,
-                        uint32_t* acts = nullptr, double* loss_zero = nullptr);
-size_t nrc_tc_bwd_bytes();
-void nrc_backward_tc_dev(aqua_ctx* ctx, const void* img, const float* Y, const float* T, int n, float inv_count,
-                         const uint32_t* acts, uint32_t* deltas, uint32_t* d6, double* loss, uint32_t* err);
-// Weight gradients of one training batch on tcgen05: per-chunk partials
-// (chunk-major, kNrcParams each) for the Adam kernel; returns the chunk count.
-int nrc_wgrad_tc_dev(aqua_ctx* ctx, const uint16_t* X, const uint32_t* acts, const uint32_t* deltas,
-                     const uint32_t* d6, int n, float* partial, uint32_t* err);
+// Both tcgen05 weight images: of w (training) and of inf (inference).
+void nrc_pack_tc(aqua_ctx* ctx, const float* w, const float* inf, void* img_w, void* img_inf);
+void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n, float* out, uint32_t* err);
+// One training batch on tcgen05: partial gradients (kNrcParams each) and loss
+// sums for the Adam kernel; returns how many, at most nrc_train_tc_max_partials.
+int nrc_train_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, const float* T, int n, float inv_count,
+                     float* partial, double* loss, uint32_t* err);
+int nrc_train_tc_max_partials(const aqua_ctx* ctx);
 // Throws when a tcgen05 launch since the last check gave up waiting (syncs the stream).
 void nrc_check_tc(aqua_ctx* ctx, NrcNet& net);
 

@@ -311,22 +311,41 @@ __global__ void __launch_bounds__(128) k_nrc_wgrad(const uint32_t* __restrict__ 
 }
 
 // ---------------------------------------------------------------- Adam
-// Kingma & Ba 2015. The gradient of parameter p is the sum of the chunk
-// partials in chunk order (deterministic).
-// With img_w non-null the new weights also go straight into the tcgen05
-// weight images (forward images of w and of the inference weights, backward
-// image of w), so no packing launch follows the step.
-__global__ void k_nrc_adam(const float* __restrict__ partial, int chunks, float* __restrict__ w,
-                           float* __restrict__ m, float* __restrict__ v, float* __restrict__ grad, float lr,
-                           float b1, float b2, float eps, float c1, float c2, float* __restrict__ ema,
-                           float ema_decay, uint8_t* __restrict__ img_w, uint8_t* __restrict__ img_inf,
-                           uint8_t* __restrict__ img_bwd) {
+// Kingma & Ba 2015. The gradient of parameter p is the sum of the partials
+// in a fixed order (deterministic): a block takes 32 parameters, warp j adds
+// partials j, j + 8, ... and the eight sums are added in order. (One thread
+// per parameter walked up to 64 partials alone: 81 blocks and a serial chain
+// of loads, 8 us at 64 partials.) losses, when given, are summed by block 0
+// into *loss. With img_w non-null the new weights also go straight into the
+// tcgen05 weight images (of w and of the inference weights), so no packing
+// launch follows the step.
+constexpr int kAdamWarps = 8;
+
+__global__ void __launch_bounds__(32 * kAdamWarps)
+    k_nrc_adam(const float* __restrict__ partial, int chunks, float* __restrict__ w, float* __restrict__ m,
+               float* __restrict__ v, float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1,
+               float c2, float* __restrict__ ema, float ema_decay, uint8_t* __restrict__ img_w,
+               uint8_t* __restrict__ img_inf, const double* __restrict__ losses, double* __restrict__ loss) {
+    __shared__ float s_sum[kAdamWarps][32];
     grid_dep_wait();
     grid_dep_launch();
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kNrcParams) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int p = (int)blockIdx.x * 32 + lane;
+    float part = 0.0f;
+    if (p < kNrcParams)
+        for (int k = warp; k < chunks; k += kAdamWarps) part += __ldcg(partial + (size_t)k * kNrcParams + p);
+    s_sum[warp][lane] = part;
+    if (losses && blockIdx.x == 0 && warp == 1) {
+        double sum = 0.0;
+        for (int k = lane; k < chunks; k += 32) sum += __ldcg(losses + k);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if (lane == 0) *loss = sum;
+    }
+    __syncthreads();
+    if (warp != 0 || p >= kNrcParams) return;
     float g = 0.0f;
-    for (int k = 0; k < chunks; ++k) g += __ldcg(partial + (size_t)k * kNrcParams + p);
+#pragma unroll
+    for (int j = 0; j < kAdamWarps; ++j) g += s_sum[j][lane];
     grad[p] = g;
     float mm = b1 * m[p] + (1.0f - b1) * g;
     float vv = b2 * v[p] + (1.0f - b2) * g * g;
@@ -344,10 +363,8 @@ __global__ void k_nrc_adam(const float* __restrict__ partial, int chunks, float*
         uint32_t fwd;
         int32_t bwd;
         nrc_tc_param_offsets(p, fwd, bwd);
-        const __nv_bfloat16 b = __float2bfloat16_rn(wn);
-        *reinterpret_cast<__nv_bfloat16*>(img_w + fwd) = b;
+        *reinterpret_cast<__nv_bfloat16*>(img_w + fwd) = __float2bfloat16_rn(wn);
         *reinterpret_cast<__nv_bfloat16*>(img_inf + fwd) = __float2bfloat16_rn(inf);
-        if (bwd >= 0) *reinterpret_cast<__nv_bfloat16*>(img_bwd + bwd) = b;
     }
 }
 
@@ -414,7 +431,7 @@ void nrc_alloc(aqua_ctx* ctx, NrcNet& net) {
     size_t o_w = take(4 * kNrcParams), o_m = take(4 * kNrcParams), o_v = take(4 * kNrcParams),
            o_g = take(4 * kNrcParams), o_f = take(8 * kFragFwd), o_b = take(8 * kFragBwd), o_l = take(64),
            o_e = take(4 * kNrcParams), o_fi = take(8 * kFragFwd), o_tc = take(nrc_tc_weight_bytes()),
-           o_tw = take(nrc_tc_weight_bytes()), o_tb = take(nrc_tc_bwd_bytes());
+           o_tw = take(nrc_tc_weight_bytes());
     dev_alloc(ctx, net.block, off);
     char* b = (char*)net.block.ptr;
     net.w = (float*)(b + o_w);
@@ -428,7 +445,6 @@ void nrc_alloc(aqua_ctx* ctx, NrcNet& net) {
     net.frag_inf = (uint2*)(b + o_fi);
     net.img_tc = (uint8_t*)(b + o_tc);
     net.img_tc_w = (uint8_t*)(b + o_tw);
-    net.img_tc_bwd = (uint8_t*)(b + o_tb);
     net.tc_err = (uint32_t*)(b + o_l + 8);  // next to the loss: one read-back carries both
     AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 4, ctx->stream));
 }
@@ -465,7 +481,7 @@ static void nrc_pack_frags(aqua_ctx* ctx, NrcNet& net) {
 void nrc_pack(aqua_ctx* ctx, NrcNet& net) {
     nrc_pack_frags(ctx, net);
     if (net.forward_tc)
-        nrc_pack_tc(ctx, net.w, net.ema_decay > 0.0f ? net.ema : net.w, net.img_tc_w, net.img_tc, net.img_tc_bwd);
+        nrc_pack_tc(ctx, net.w, net.ema_decay > 0.0f ? net.ema : net.w, net.img_tc_w, net.img_tc);
 }
 
 void nrc_set_weights(aqua_ctx* ctx, NrcNet& net, const float* host_w) {
@@ -496,15 +512,17 @@ void nrc_forward_dev(aqua_ctx* ctx, NrcNet& net, const uint16_t* X, int n, float
     AQ_CUDA(cudaGetLastError());
 }
 
+// Training scratch: the tcgen05 step keeps one partial gradient and loss per
+// CTA; the mma.sync step keeps every row's activations and deltas too.
 static void ensure_train(aqua_ctx* ctx, NrcNet& net, int n) {
     if (net.train.ptr && net.train_rows >= n) return;
     dev_free(net.train);
-    int rows = std::max(n, 1024);
-    int chunks = (rows + kWgChunk - 1) / kWgChunk;
+    const size_t rows = net.forward_tc ? 0 : (size_t)std::max(n, 1024);
+    const size_t chunks = net.forward_tc ? (size_t)nrc_train_tc_max_partials(ctx) : (rows + kWgChunk - 1) / kWgChunk;
     size_t off = 0;
     auto take = [&](size_t b) { size_t o = off; off = rup(off + b, 256); return o; };
-    size_t o_y = take(12 * (size_t)rows), o_a = take(5 * 128 * (size_t)rows), o_d = take(5 * 128 * (size_t)rows),
-           o_6 = take(32 * (size_t)rows), o_p = take(4 * (size_t)kNrcParams * chunks);
+    size_t o_y = take(12 * rows), o_a = take(5 * 128 * rows), o_d = take(5 * 128 * rows), o_6 = take(32 * rows),
+           o_p = take(4 * (size_t)kNrcParams * chunks), o_l = take(8 * chunks);
     dev_alloc(ctx, net.train, off);
     char* b = (char*)net.train.ptr;
     net.ty = (float*)(b + o_y);
@@ -512,45 +530,40 @@ static void ensure_train(aqua_ctx* ctx, NrcNet& net, int n) {
     net.deltas = (uint32_t*)(b + o_d);
     net.d6 = (uint32_t*)(b + o_6);
     net.partial = (float*)(b + o_p);
-    net.train_rows = rows;
+    net.losses = (double*)(b + o_l);
+    net.train_rows = net.forward_tc ? INT32_MAX : (int)rows;
 }
 
 void nrc_train_step_dev(aqua_ctx* ctx, NrcNet& net, const uint16_t* X, const float* target, int n) {
     if (n <= 0) return;
     ensure_train(ctx, net, n);
     cudaStream_t st = ctx->stream;
-    const uint32_t* Xw = reinterpret_cast<const uint32_t*>(X);
-    int g = nrc_grid(ctx, n);
-    // On tcgen05 the four launches of a step (and of consecutive steps) are
-    // chained (programmatic dependent launch); the forward pass zeroes the
-    // loss word and Adam writes the next step's weight images.
+    const float inv_count = 1.0f / (float)(n * kNrcOut);
+    int chunks;
+    // On tcgen05 a step is two launches, chained (programmatic dependent
+    // launch) to each other and to the next step's; Adam writes the next
+    // step's weight images.
     if (net.forward_tc) {
-        nrc_forward_tc_dev(ctx, net.img_tc_w, X, n, net.ty, net.tc_err, net.acts, net.loss);
+        chunks = nrc_train_tc_dev(ctx, net.img_tc_w, X, target, n, inv_count, net.partial, net.losses, net.tc_err);
     } else {
+        const uint32_t* Xw = reinterpret_cast<const uint32_t*>(X);
+        const int g = nrc_grid(ctx, n);
         k_nrc_forward<true><<<g, 128, 0, st>>>(Xw, n, net.frag, net.ty, net.acts);
         AQ_CUDA(cudaMemsetAsync(net.loss, 0, 8, st));
-    }
-    if (net.forward_tc)
-        nrc_backward_tc_dev(ctx, net.img_tc_bwd, net.ty, target, n, 1.0f / (float)(n * kNrcOut), net.acts,
-                            net.deltas, net.d6, net.loss, net.tc_err);
-    else
-        k_nrc_backward<<<g, 128, 0, st>>>(net.ty, target, n, 1.0f / (float)(n * kNrcOut), net.fragT, net.acts,
-                                          net.deltas, net.d6, net.loss);
-    int chunks;
-    if (net.forward_tc) {
-        chunks = nrc_wgrad_tc_dev(ctx, X, net.acts, net.deltas, net.d6, n, net.partial, net.tc_err);
-    } else {
+        k_nrc_backward<<<g, 128, 0, st>>>(net.ty, target, n, inv_count, net.fragT, net.acts, net.deltas, net.d6,
+                                          net.loss);
         chunks = (n + kWgChunk - 1) / kWgChunk;
         k_nrc_wgrad<<<dim3(chunks, 6), 128, 0, st>>>(Xw, net.acts, net.deltas, net.d6, n, net.partial);
     }
     net.step++;
     float c1 = 1.0f - powf(net.beta1, (float)net.step), c2 = 1.0f - powf(net.beta2, (float)net.step);
-    launch_chained(k_nrc_adam, dim3((kNrcParams + 255) / 256), dim3(256), 0, st, (const float*)net.partial, chunks,
-                   net.w, net.m, net.v, net.grad, net.lr, net.beta1, net.beta2, net.eps, c1, c2, net.ema,
-                   net.ema_decay, net.forward_tc ? net.img_tc_w : nullptr, net.img_tc, net.img_tc_bwd);
+    launch_chained(k_nrc_adam, dim3((kNrcParams + 31) / 32), dim3(32 * kAdamWarps), 0, st, (const float*)net.partial,
+                   chunks, net.w, net.m, net.v, net.grad, net.lr, net.beta1, net.beta2, net.eps, c1, c2, net.ema,
+                   net.ema_decay, net.forward_tc ? net.img_tc_w : nullptr, net.img_tc,
+                   net.forward_tc ? (const double*)net.losses : nullptr, net.loss);
     if (!net.forward_tc) nrc_pack_frags(ctx, net);
     AQ_CUDA(cudaGetLastError());
-    net.launches += net.forward_tc ? 4 : 6;
+    net.launches += net.forward_tc ? 2 : 6;
 }
 
 void nrc_check_tc(aqua_ctx* ctx, NrcNet& net) {

@@ -42,16 +42,12 @@
 namespace aq {
 
 constexpr int kTcRows = 128;                      // rows per tile (MMA M)
-constexpr int kTcGroups = 4;                      // warpgroups (tiles in flight) per CTA, training kernels
-constexpr int kTcThreads = 128 * kTcGroups;
 constexpr int kTcTileBytes = kTcRows * 64 * 2;    // 16 KB per input or activation tile
 constexpr int kTcLayerBytes = kNrcTcLayerBytes;  // 8 KB hidden-layer weights
 constexpr int kTcOutRows = kNrcTcOutRows;        // output layer padded to N = 16 (3 used)
 constexpr int kTcOutBytes = kTcOutRows * 64 * 2;  // 2 KB
 constexpr int kTcWeightBytes = 5 * kTcLayerBytes + kTcOutBytes;  // 42 KB
-constexpr uint32_t kTcGroupCols = 128;            // accumulator 64 + activations 32, rounded up
-constexpr uint32_t kTcActCol = 64;                // activation columns within a group
-constexpr uint32_t kTcTmemCols = kTcGroupCols * kTcGroups;  // a power of two >= 32
+constexpr uint32_t kTcTmemCols = 512;              // a power of two >= 32
 constexpr uint32_t kTcWaitLimit = 1u << 22;       // try_wait rounds before a wait gives up
 // Inference: five groups (tiles in flight; four measured 9% slower),
 // accumulators at columns 64 g, activations after all accumulators at
@@ -69,20 +65,17 @@ static_assert(kTcWeightBytes % 1024 == 0 && kTcTileBytes % 1024 == 0, "tiles sta
 // Byte offset of element (r, k) in an R-row operand tile.
 __host__ __device__ constexpr uint32_t tc_offset(int rows, int r, int k) { return nrc_tc_offset(rows, r, k); }
 
-// All three weight images from the FP32 weights w and the inference
-// weights inf (nrc_tc_param_offsets; the caller zeroes the padding first):
-// forward images of w (training) and of inf (inference), backward image of w.
+// Both weight images from the FP32 weights w (training) and the inference
+// weights inf (nrc_tc_param_offsets; the caller zeroes the padding first).
 __global__ void k_nrc_pack_tc(const float* __restrict__ w, const float* __restrict__ inf, uint8_t* __restrict__ img_w,
-                              uint8_t* __restrict__ img_inf, uint8_t* __restrict__ img_bwd) {
+                              uint8_t* __restrict__ img_inf) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;  // one parameter
     if (p >= kNrcParams) return;
     uint32_t fwd;
     int32_t bwd;
     nrc_tc_param_offsets(p, fwd, bwd);
-    const __nv_bfloat16 b = __float2bfloat16_rn(w[p]);
-    *reinterpret_cast<__nv_bfloat16*>(img_w + fwd) = b;
+    *reinterpret_cast<__nv_bfloat16*>(img_w + fwd) = __float2bfloat16_rn(w[p]);
     *reinterpret_cast<__nv_bfloat16*>(img_inf + fwd) = __float2bfloat16_rn(inf[p]);
-    if (bwd >= 0) *reinterpret_cast<__nv_bfloat16*>(img_bwd + bwd) = b;
 }
 
 // ---------------------------------------------------------------- PTX wrappers
@@ -214,12 +207,10 @@ __device__ __forceinline__ uint32_t relu_pack2(uint32_t lo, uint32_t hi) {
 
 // ---------------------------------------------------------------- kernel
 // X (through `xmap`): n rows x 64 bf16; out: n x 3 fp32; err: set to 1 when a
-// wait expired. acts (training, may be null): the hidden activations H1..H5
-// as bf16 rows, acts[l][row][64], for the backward pass.
+// wait expired.
 __global__ void __launch_bounds__(kTcFwdThreads, 1)
     k_nrc_forward_tc(const __grid_constant__ CUtensorMap xmap, int n, const uint4* __restrict__ wimg,
-                     float* __restrict__ out, uint32_t* __restrict__ err, uint4* __restrict__ acts,
-                     double* __restrict__ loss_zero) {
+                     float* __restrict__ out, uint32_t* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bar_in[kTcFwdGroups], bar_mma[kTcFwdGroups];
     __shared__ uint32_t tmem_base_slot;
@@ -233,7 +224,6 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
 
     grid_dep_wait();  // the weights and inputs come from the kernels before
     grid_dep_launch();
-    if (loss_zero && blockIdx.x == 0 && tid == 0) *loss_zero = 0.0;  // the training step's loss word
     for (int i = tid; i < kTcWeightBytes / 16; i += kTcFwdThreads) reinterpret_cast<uint4*>(sbase)[i] = __ldcg(wimg + i);
     if (tid < kTcFwdGroups) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&bar_in[tid])) : "memory");
@@ -331,13 +321,6 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
                     for (int c = 0; c < 32; ++c) a[c] = relu_pack2(r[2 * c], r[2 * c + 1]);
                     AQ_TC_ST16(tact + lanes + 0u, (a + 0));
                     AQ_TC_ST16(tact + lanes + 16u, (a + 16));
-                    const int grow = tile * kTcRows + row;
-                    if (acts && grow < n) {
-                        uint4* dst = acts + ((size_t)l * (size_t)n + (size_t)grow) * 8;
-#pragma unroll
-                        for (int q4 = 0; q4 < 8; ++q4)
-                            dst[q4] = make_uint4(a[4 * q4], a[4 * q4 + 1], a[4 * q4 + 2], a[4 * q4 + 3]);
-                    }
                     tc_wait_st();
                 } else {
                     uint32_t r[16];
@@ -373,20 +356,64 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
     }
 }
 
-// ---------------------------------------------------------------- backward
-// The training step's backward pass on the same machinery (relative L2 loss
-// of Mueller et al. 2021 with y^2 held constant, as k_nrc_backward). Per
-// 128-row tile: dY (16 columns, 3 used) from Y and the targets becomes the
-// A operand in TMEM; dH5 = dY x W6 (one K = 16 MMA); then for layers 5..1
-// the epilogue masks dH with ReLU'(H) read from the stored activations,
-// rounds to bf16, writes delta_l for the weight gradients and, above layer
-// 1, stores it back to TMEM as the A operand of dH_{l-1} = delta_l x W_l.
-// Weight image (rows = N = 64 inputs, K = outputs): W6^T (K = 16) then
-// W5^T..W2^T (K = 64).
-constexpr int kTcBwdW6Bytes = kNrcTcBwdW6Bytes;                    // 2 KB
-constexpr int kTcBwdBytes = kTcBwdW6Bytes + 4 * kTcLayerBytes;      // 34 KB
-constexpr int kTcBwdSmemBytes = std::max(kTcBwdBytes + 1024, 120 * 1024);  // one CTA per SM
+// ---------------------------------------------------------------- training
+// One optimisation step's forward pass, backward pass and weight gradients in
+// one persistent kernel (relative L2 loss of Mueller et al. 2021 with y^2 held
+// constant, as k_nrc_backward). Separate kernels wrote the five activations
+// and deltas of every row to memory and read them back, 3.6 KB per row, and
+// the step was bound by that traffic and the launches' ramps; here a row's
+// activations live in shared memory from its forward pass to its weight
+// gradients, and a row costs its 128 B of input and 12 B of target.
+//
+// A CTA holds the forward weight image (42 KB) and runs two groups of 256
+// threads, each with a 128-row tile in flight: five 16 KB buffers (the input
+// and H1..H4; H5 takes the input's place) and dY (4 KB). One more warp issues
+// every MMA:
+//   steps 0-5   layer l's accumulator = H_{l-1} W_l^T
+//   step 6      dH5 = dY W6, and dW6^T += H5^T dY
+//   steps 7-10  dH_l = delta_{l+1} W_{l+1}, and dW_{l+1} += delta_{l+1}^T H_l
+//   step 11     dW1 += delta1^T X
+// and a group's threads (two per row, 32 columns each) turn an accumulator
+// into the next operand: ReLU and bf16 for H_l, the loss gradient for dY,
+// ReLU' for delta_l, which overwrites H_l once the MMAs that read it are done.
+// While one group is in its epilogue the tensor core works for the other. The
+// input comes in by TMA twice, before layer 1 and, into the buffer that
+// delta5 leaves, for dW1; the next tile's input is fetched into delta4's.
+//
+// All operands share one storage: element (row, feature) of a tile at
+// (feature / 8) slice + row 16 + (feature % 8) 2 bytes. Read with 128-byte
+// steps between 8-row groups it is K-major over features (the layer MMAs' A),
+// read with 128-byte steps along K it is MN-major with K = rows (the weight
+// gradients' A and B); likewise one weight image serves W_l^T and W_l.
+// The weight gradients of all layers accumulate in TMEM over every tile of
+// the CTA (336 columns; a layer's 64 outputs are lanes 0-63 of an M = 128 MMA
+// whose upper rows read, and ignore, the neighbouring buffer) and leave once,
+// as this CTA's partial for the Adam kernel. One thread issues all MMAs, so
+// the accumulations of both groups are ordered and a step is reproducible.
+//
+// Bound: the chain of eleven dependent MMA -> epilogue steps per tile, about
+// 1400 cycles each, with two tiles in flight (the activations fill shared
+// memory); without any weight-gradient MMA 250,007 rows take 73 us instead of
+// 78. Measured (one step with Adam, device time): 250,007 rows 302 -> 78 us,
+// 65,536 rows 85 -> 36 us, 16,384 rows 40 -> 25 us.
+//
+// Every wait is bounded: a wait that expires raises a flag that ends all
+// others, and TMEM is freed on every path.
+constexpr int kTrGroups = 2;
+constexpr int kTrThreads = 256 * kTrGroups + 32;   // two threads per row, and the issuing warp
+// Bytes between the 8-feature slices of a tile and of a layer's weights.
+// (16 bytes of padding, which put the slices on different banks for the
+// MN-major reads, changed nothing.)
+constexpr uint32_t kTrSlice = kTcRows * 16, kTrWSlice = 64 * 16, kTrW6Slice = kTcOutRows * 16;
+constexpr int kTrDyBytes = 2 * kTrSlice;           // dY, 16 columns (3 used)
+constexpr int kTrGroupBytes = 5 * kTcTileBytes;
+// dY of both groups, the groups' buffers, then the weights: an M = 128 weight
+// gradient reads up to 16 KB past its buffer, which stays inside.
+constexpr int kTrSmemBytes = kTrGroups * (kTrDyBytes + kTrGroupBytes) + kTcWeightBytes + 1024;
+constexpr uint32_t kTrW6Col = 320, kTrAccCol = 352;  // dW1..dW5 at 64 L, dW6^T, the groups' accumulators
 constexpr float kTcLossEps = 0.01f;
+static_assert(kTrSmemBytes <= 227 * 1024, "shared memory per CTA");
+static_assert(kTrAccCol + 64 * kTrGroups <= 512, "TMEM columns");
 
 __device__ __forceinline__ uint32_t pack2_rn(float lo, float hi) {
     uint32_t d;
@@ -394,165 +421,387 @@ __device__ __forceinline__ uint32_t pack2_rn(float lo, float hi) {
     return d;
 }
 
-#define AQ_TC_ST8(taddr, r)                                                                            \
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr), \
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])  \
-                 : "memory")
+// 0xffff in each half of a bf16 pair that is above zero.
+__device__ __forceinline__ uint32_t positive2(uint32_t h) {
+    __nv_bfloat162 a;
+    *reinterpret_cast<uint32_t*>(&a) = h;
+    return __hgt2_mask(a, __floats2bfloat162_rn(0.0f, 0.0f));
+}
 
-// Y, T: n x 3 fp32 (outputs, targets); acts: H1..H5 bf16 rows; deltas:
-// delta_1..delta_5 bf16 rows; d6: dY as 16 bf16 per row; loss: += sum of
-// the per-element losses; err: 1 when a wait expired.
-__global__ void __launch_bounds__(kTcThreads, 1)
-    k_nrc_backward_tc(const float* __restrict__ Y, const float* __restrict__ T, int n, float inv_count,
-                      const uint4* __restrict__ wimg, const uint4* __restrict__ acts, uint4* __restrict__ deltas,
-                      uint4* __restrict__ d6, double* __restrict__ loss, uint32_t* __restrict__ err) {
+// Descriptors from a shared address >> 4 (no swizzle). K-major: `lbo` bytes
+// between groups of 8 along K, 128 between groups of 8 rows of the result.
+// MN-major: 128 between groups of 8 along K, `sbo` between groups of 8 rows.
+__device__ __forceinline__ uint64_t desc_k(uint32_t a, uint32_t lbo) {
+    return (uint64_t)(a | ((lbo >> 4) << 16)) | ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
+}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t a, uint32_t sbo) {
+    return (uint64_t)(a | ((128u >> 4) << 16)) | ((uint64_t)((sbo >> 4) | (1u << 14)) << 32);
+}
+
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
+// tc_mma by the elected lane of a warp that runs converged.
+__device__ __forceinline__ void tc_issue(bool lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead));
+}
+constexpr uint32_t kIdescAMn = 1u << 15, kIdescBMn = 1u << 16;  // A, B are MN-major
+
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
+}
+
+// Bounded wait that also ends when another wait of the CTA has expired.
+__device__ __forceinline__ bool mbar_wait_or(uint32_t mbar, uint32_t parity, volatile uint32_t* failed) {
+    for (uint32_t it = 0; it < kTcWaitLimit; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(mbar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((it & 15u) == 15u && *failed) return false;
+    }
+    *failed = 1u;
+    return false;
+}
+
+// T: n x 3 targets; partial: one kNrcParams vector per CTA; loss: one sum of
+// per-element losses per CTA; err: set to 1 when a wait expired.
+__global__ void __launch_bounds__(kTrThreads, 1)
+    k_nrc_train_tc(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ T, int n, float inv_count,
+                   const uint4* __restrict__ wimg, float* __restrict__ partial, double* __restrict__ loss,
+                   uint32_t* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bar_mma[kTcGroups];
-    __shared__ uint32_t tmem_base_slot;
+    __shared__ __align__(8) uint64_t bars[5 * kTrGroups];
+    __shared__ float s_loss[8 * kTrGroups];
+    __shared__ uint32_t tmem_slot, s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = warp >> 2, q = warp & 3, gt = tid & 127;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* sbase = smem_raw + (base - smem_u32(smem_raw));
-    grid_dep_wait();
-    grid_dep_launch();
-    for (int i = tid; i < kTcBwdBytes / 16; i += kTcThreads) reinterpret_cast<uint4*>(sbase)[i] = __ldcg(wimg + i);
-    if (tid < kTcGroups)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&bar_mma[tid])) : "memory");
-    if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    constexpr uint32_t kBuf0 = kTrGroups * kTrDyBytes, kW0 = kBuf0 + kTrGroups * kTrGroupBytes;
+    // Barriers of group g: input landed, input landed again, operand ready
+    // (8 warps), accumulator complete, weight-gradient MMAs complete.
+    enum { kX = 0, kR = 1, kReady = 2, kAcc = 3, kWg = 4 };
+    auto bar = [&](int g, int k) { return smem_u32(&bars[5 * g + k]); };
+
+    if (tid < 5 * kTrGroups)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&bars[tid])),
+                     "r"(tid % 5 == kReady ? 8u : 1u)
+                     : "memory");
+    if (tid == 0) {
+        s_failed = 0u;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&xmap)) : "memory");
+    }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                         smem_u32(&tmem_base_slot)),
-                     "r"(kTcTmemCols)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    grid_dep_wait();  // the weights and inputs come from the kernels before
+    grid_dep_launch();
+    for (int i = tid; i < kTcWeightBytes / 16; i += kTrThreads)
+        reinterpret_cast<uint4*>(sbase + kW0)[i] = __ldcg(wimg + i);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_base_slot + (uint32_t)g * kTcGroupCols;
-    const uint32_t tact = tmem + kTcActCol;
-    const uint32_t lanes = (uint32_t)(q * 32) << 16;
-    const uint32_t mb = smem_u32(&bar_mma[g]);
-    const int bar_id = 1 + g;
+
+    // All 512 columns were allocated, so they start at 0; the constant keeps
+    // the issuing warp's TMEM addresses uniform.
+    constexpr uint32_t tmem = 0u;
+    if (tid == 0 && tmem_slot != 0u) s_failed = 1u;
     const int tiles = (n + kTcRows - 1) / kTcRows;
-    const int row = q * 32 + lane;
-    uint32_t ph = 0, mma_par = 0;
-    bool fail = false, pending = false;
+    const int stride = (int)gridDim.x * kTrGroups;
     float lsum = 0.0f;
-    for (int tile = (int)blockIdx.x + g * (int)gridDim.x; tile < tiles; tile += (int)gridDim.x * kTcGroups) {
-        const int grow = tile * kTcRows + row;
-        const bool valid = grow < n;
-        // dY of this row (columns 0..2), packed as 16 bf16.
-        float gy[3] = {0.0f, 0.0f, 0.0f};
-        if (valid) {
+
+    if (warp == 8 * kTrGroups) {
+        // ------------------------------------------------ the issuing warp
+        // All lanes run it with warp-uniform values, so that addresses and
+        // descriptors live in uniform registers, and one lane issues: code
+        // run by a single lane moved four registers to the uniform file for
+        // every MMA, 110 cycles each, and bound the kernel (250,007 rows
+        // 120 us).
+        const bool lead = elect_one();
+        const uint32_t idesc = tc_idesc(kTcRows, 64);
+        // Low descriptor words: the groups' buffers (input, H1..H4), dY, weights.
+        uint32_t b[kTrGroups][5], dy[kTrGroups];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                float y = __ldcg(Y + (size_t)grow * 3 + c), t = __ldcg(T + (size_t)grow * 3 + c);
-                float den = y * y + kTcLossEps, d = y - t;
-                lsum += d * d / den;
-                gy[c] = 2.0f * d / den * inv_count;
-            }
-        }
-        uint32_t a6[8] = {pack2_rn(gy[0], gy[1]), pack2_rn(gy[2], 0.0f), 0u, 0u, 0u, 0u, 0u, 0u};
-        if (valid) {
-            d6[(size_t)grow * 2] = make_uint4(a6[0], a6[1], 0u, 0u);
-            d6[(size_t)grow * 2 + 1] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        AQ_TC_ST8(tact + lanes, a6);
-        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-        tc_fence_before();
-        group_sync(bar_id);  // dY is in TMEM before the first MMA
-        for (int l = 4; l >= 0; --l) {  // this MMA gives dH of hidden layer l + 1
-            if (gt == 0) {
-                tc_fence_after();
-                const uint32_t idesc = tc_idesc(kTcRows, 64);
-                if (l == 4) {
-                    tc_mma_ts(tmem, tact, tc_desc(base, 64 * 16), idesc, 0u);
-                } else {
-                    const uint32_t b0 = base + kTcBwdW6Bytes + (uint32_t)(3 - l) * kTcLayerBytes;
+        for (int g = 0; g < kTrGroups; ++g) {
+            dy[g] = (base + (uint32_t)g * kTrDyBytes) >> 4;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma_ts(tmem, tact + (uint32_t)k * 8u, tc_desc(b0 + (uint32_t)k * 2u * (64 * 16), 64 * 16),
-                                  idesc, k > 0 ? 1u : 0u);
+            for (int k = 0; k < 5; ++k)
+                b[g][k] = (base + kBuf0 + (uint32_t)g * kTrGroupBytes + (uint32_t)k * kTcTileBytes) >> 4;
+        }
+        const uint32_t w0 = (base + kW0) >> 4;
+        uint32_t par = 0;      // parity of kX and kR (one phase per tile)
+        uint32_t par_rdy = 0;  // bit g: parity of the group's kReady
+        uint32_t sums = 0;     // 1 once the dW accumulators hold sums (group 0 starts them)
+        bool ok = true;
+        for (int t0 = (int)blockIdx.x; t0 < tiles; t0 += stride) {
+#pragma unroll
+            for (int step = 0; step < 12; ++step) {
+#pragma unroll
+                for (int g = 0; g < kTrGroups; ++g) {
+                    if (t0 + g * (int)gridDim.x >= tiles || !ok) break;
+                    const uint32_t acc = kTrAccCol + 64u * (uint32_t)g;
+                    if (step == 0) {
+                        ok = mbar_wait_or(bar(g, kX), par, &s_failed);
+                    } else {
+                        ok = mbar_wait_or(bar(g, kReady), (par_rdy >> g) & 1u, &s_failed);
+                        par_rdy ^= 1u << g;
+                    }
+                    if (step == 11) ok = ok && mbar_wait_or(bar(g, kR), par, &s_failed);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    // The layer MMAs: A is K-major over features.
+                    constexpr uint32_t kStep = 2 * kTrSlice / 16, kWStep = 2 * kTrWSlice / 16, kW6Step = 2 * kTrW6Slice / 16;
+                    if (step < 5) {  // H_{step+1}, from buffer `step` (0: the input)
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k)
+                            tc_issue(lead, acc, desc_k(b[g][step] + k * kStep, kTrSlice),
+                                     desc_k(w0 + (uint32_t)step * (kTcLayerBytes / 16) + k * kWStep, kTrWSlice), idesc, k > 0);
+                    } else if (step == 5) {  // the outputs, from H5 in buffer 0
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k)
+                            tc_issue(lead, acc, desc_k(b[g][0] + k * kStep, kTrSlice),
+                                     desc_k(w0 + 5u * (kTcLayerBytes / 16) + k * kW6Step, kTrW6Slice),
+                                     tc_idesc(kTcRows, kTcOutRows), k > 0);
+                    } else if (step == 6) {  // dH5 = dY W6, K = 16 outputs
+                        tc_issue(lead, acc, desc_k(dy[g], kTrSlice), desc_mn(w0 + 5u * (kTcLayerBytes / 16), kTrW6Slice),
+                                 idesc | kIdescBMn, 0u);
+                    } else if (step < 11) {  // dH_{11-step}, from delta_{12-step}
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k)
+                            tc_issue(lead, acc, desc_k(b[g][(12 - step) % 5] + k * kStep, kTrSlice),
+                                     desc_mn(w0 + (uint32_t)(11 - step) * (kTcLayerBytes / 16) + k * 16u, kTrWSlice),
+                                     idesc | kIdescBMn, k > 0);
+                    }
+                    if (step < 11 && lead) tc_commit(bar(g, kAcc));
+                    // The weight gradients: K = rows, both operands MN-major.
+                    const uint32_t add = g > 0 ? 1u : sums;
+                    if (step == 6) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k)
+                            tc_issue(lead, kTrW6Col, desc_mn(b[g][0] + k * 16u, kTrSlice),
+                                     desc_mn(dy[g] + k * 16u, kTrSlice),
+                                     tc_idesc(kTcRows, kTcOutRows) | kIdescAMn | kIdescBMn, k > 0 ? 1u : add);
+                    } else if (step > 6) {  // dW_{12-step}: delta_{12-step} with H_{11-step} (step 11: the input)
+#pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k)
+                            tc_issue(lead, 64u * (uint32_t)(11 - step),
+                                     desc_mn(b[g][(12 - step) % 5] + k * 16u, kTrSlice),
+                                     desc_mn(b[g][11 - step] + k * 16u, kTrSlice),
+                                     idesc | kIdescAMn | kIdescBMn, k > 0 ? 1u : add);
+                    }
+                    if (step >= 6 && lead) tc_commit(bar(g, kWg));
                 }
-                tc_commit(mb);
-                pending = true;
-                mma_par = ph;
             }
-            bool ok = mbar_wait(mb, ph);
-            ph ^= 1u;
-            ok = __all_sync(0xffffffffu, ok);
-            if (gt == 0 && ok) pending = false;
+            if (!ok) break;
+            sums = 1u;
+            par ^= 1u;
+#pragma unroll
+            for (int g = 0; g < kTrGroups; ++g) {  // the next input lies where delta4 was
+                const uint32_t last = b[g][4];
+#pragma unroll
+                for (int k = 4; k > 0; --k) b[g][k] = b[g][k - 1];
+                b[g][0] = last;
+            }
+        }
+    } else {
+        // ------------------------------------------------ a group's rows
+        const int g = warp >> 3, q = warp & 3, gt = tid & 255;
+        const uint32_t half = (uint32_t)(warp >> 2) & 1u;  // columns 32 half .. 32 half + 31
+        const uint32_t row = (uint32_t)(q * 32 + lane);  // TMEM lane = tile row
+        const uint32_t lanes = (uint32_t)(q * 32) << 16;
+        const uint32_t acc = tmem + kTrAccCol + 64u * (uint32_t)g + 32u * half + lanes;
+        const uint32_t b0 = base + kBuf0 + (uint32_t)g * kTrGroupBytes;
+        uint8_t* gbuf = sbase + kBuf0 + (size_t)g * kTrGroupBytes;
+        uint32_t ph_acc = 0, ph_wg = 0, o = 0;
+        bool ok = true, wg_open = false;  // wg_open: the last tile's dW1 not yet waited for
+        auto wait_acc = [&]() {
+            ok = ok && mbar_wait_or(bar(g, kAcc), ph_acc, &s_failed);
+            ph_acc ^= 1u;
+            ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld is warp-collective
             tc_fence_after();
-            if (ok) {
-                uint32_t r[64], a[32];
-                AQ_TC_LD16(tmem + lanes + 0u, (r + 0));
-                AQ_TC_LD16(tmem + lanes + 16u, (r + 16));
-                AQ_TC_LD16(tmem + lanes + 32u, (r + 32));
-                AQ_TC_LD16(tmem + lanes + 48u, (r + 48));
+            return ok;
+        };
+        auto wait_wg = [&]() {
+            ok = ok && mbar_wait_or(bar(g, kWg), ph_wg, &s_failed);
+            ph_wg ^= 1u;
+            ok = __all_sync(0xffffffffu, ok);
+            return ok;
+        };
+        auto ready = [&]() {  // this warp's rows of the next operand are in place
+            fence_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(g, kReady));
+        };
+        auto half_row = [&](uint32_t k) {  // this thread's 32 features in buffer k, 8 every 2048 bytes
+            return gbuf + (o + k) % 5u * (uint32_t)kTcTileBytes + half * 4u * kTrSlice + row * 16u;
+        };
+        int tile = (int)blockIdx.x + g * (int)gridDim.x;
+        if (gt == 0 && tile < tiles) tma_load_tile(&xmap, b0, bar(g, kX), tile * kTcRows);
+        for (; tile < tiles; tile += stride) {
+            const int grow = tile * kTcRows + (int)row;
+            const bool valid = grow < n;
+            float t[3] = {0.0f, 0.0f, 0.0f};
+            if (valid)
+                for (int c = 0; c < 3; ++c) t[c] = __ldcg(T + (size_t)grow * 3 + c);
+            uint32_t r[32];
+            for (uint32_t l = 0; l < 5; ++l) {  // H_{l+1} into buffer l + 1 (H5 into 0)
+                if (!wait_acc()) break;
+                if (l == 0 && wg_open) {
+                    if (!wait_wg()) break;
+                    wg_open = false;
+                }
+                AQ_TC_LD16(acc + 0u, (r + 0));
+                AQ_TC_LD16(acc + 16u, (r + 16));
                 tc_wait_ld();
-                // ReLU'(Z) from the stored activation H = ReLU(Z) in bf16.
-                uint4 h[8];
+                uint8_t* dst = half_row(l + 1);
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    h[j] = valid ? __ldcg(acts + ((size_t)l * (size_t)n + (size_t)grow) * 8 + (size_t)j) : make_uint4(0, 0, 0, 0);
+                for (uint32_t j = 0; j < 4; ++j)
+                    *reinterpret_cast<uint4*>(dst + j * kTrSlice) =
+                        make_uint4(relu_pack2(r[8 * j], r[8 * j + 1]), relu_pack2(r[8 * j + 2], r[8 * j + 3]),
+                                   relu_pack2(r[8 * j + 4], r[8 * j + 5]), relu_pack2(r[8 * j + 6], r[8 * j + 7]));
+                ready();
+            }
+            if (!ok) break;
+            if (!wait_acc()) break;
+            if (half == 0) {  // dY = dLoss / dY, columns 0..2 of 16
+                uint32_t y[16];
+                AQ_TC_LD16(acc, y);
+                tc_wait_ld();
+                float gy[3] = {0.0f, 0.0f, 0.0f};
+                if (valid) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t hw[4] = {h[j].x, h[j].y, h[j].z, h[j].w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int c = 4 * j + e;  // bf16 pair (2c, 2c + 1)
-                        float lo = __uint_as_float(r[2 * c]), hi = __uint_as_float(r[2 * c + 1]);
-                        if (!(__uint_as_float(hw[e] << 16) > 0.0f)) lo = 0.0f;
-                        if (!(__uint_as_float(hw[e] & 0xffff0000u) > 0.0f)) hi = 0.0f;
-                        a[c] = pack2_rn(lo, hi);
+                    for (int c = 0; c < 3; ++c) {
+                        const float yc = __uint_as_float(y[c]);
+                        const float den = yc * yc + kTcLossEps, d = yc - t[c];
+                        lsum += d * d / den;
+                        gy[c] = 2.0f * d / den * inv_count;
                     }
                 }
-                if (valid) {
-                    uint4* dst = deltas + ((size_t)l * (size_t)n + (size_t)grow) * 8;
+                uint8_t* dy = sbase + (size_t)g * kTrDyBytes + row * 16u;
+                *reinterpret_cast<uint4*>(dy) = make_uint4(pack2_rn(gy[0], gy[1]), pack2_rn(gy[2], 0.0f), 0u, 0u);
+                *reinterpret_cast<uint4*>(dy + kTrSlice) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            ready();
+            for (uint32_t l = 5; l >= 1; --l) {  // delta_l over H_l, in buffer l % 5
+                if (!wait_acc()) break;
+                uint8_t* dst = half_row(l);
+                uint4 h[4];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) dst[j] = make_uint4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
-                }
-                if (l > 0) {
-                    AQ_TC_ST16(tact + lanes + 0u, (a + 0));
-                    AQ_TC_ST16(tact + lanes + 16u, (a + 16));
-                    tc_wait_st();
-                }
+                for (uint32_t j = 0; j < 4; ++j) h[j] = *reinterpret_cast<const uint4*>(dst + j * kTrSlice);
+                AQ_TC_LD16(acc + 0u, (r + 0));
+                AQ_TC_LD16(acc + 16u, (r + 16));
+                tc_wait_ld();
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j)  // ReLU'(Z) from H = ReLU(Z)
+                    h[j] = make_uint4(pack2_rn(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])) & positive2(h[j].x),
+                                      pack2_rn(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])) & positive2(h[j].y),
+                                      pack2_rn(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])) & positive2(h[j].z),
+                                      pack2_rn(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])) & positive2(h[j].w));
+                if (!wait_wg()) break;  // the weight gradient that reads H_l is done
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(dst + j * kTrSlice) = h[j];
+                ready();
+                // delta5's buffer is free after step 7, delta4's after step 8.
+                if (gt == 0 && l == 4) tma_load_tile(&xmap, b0 + o * (uint32_t)kTcTileBytes, bar(g, kR), tile * kTcRows);
+                if (gt == 0 && l == 3 && tile + stride < tiles)
+                    tma_load_tile(&xmap, b0 + (o + 4u) % 5u * (uint32_t)kTcTileBytes, bar(g, kX),
+                                  (tile + stride) * kTcRows);
             }
-            tc_fence_before();
-            if (group_any(bar_id, !ok)) {
-                fail = true;
-                break;
-            }
+            if (!ok) break;
+            wg_open = true;  // dW1
+            o = (o + 4u) % 5u;
         }
-        if (fail) break;
-    }
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, o);
-    if (lane == 0 && lsum != 0.0f) atomicAdd(loss, (double)lsum);
-    if (fail && gt == 0) {
-        atomicExch(err, 1u);
-        if (pending) mbar_wait(mb, mma_par);
+        if (wg_open) wait_wg();
+        for (int k = 16; k > 0; k >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, k);
+        if (lane == 0) s_loss[warp] = lsum;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base_slot),
-                     "r"(kTcTmemCols)
-                     : "memory");
+    if (s_failed) {
+        if (tid == 0) atomicExch(err, 1u);
+        // Whatever is still in flight (TMA, MMAs) lands within these bounded waits.
+        if (tid < 5 * kTrGroups)
+            for (uint32_t it = 0; it < 2; ++it) mbar_wait(smem_u32(&bars[tid]), it);
+    } else if (warp < 8 * kTrGroups && (warp & 3) < 2) {
+        // Lanes 0..63 hold the outputs of a layer (dW6^T: the inputs), which warps 0
+        // and 1 of every four can read; the fours share the layers.
+        const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+        const int orow = (warp & 3) * 32 + lane;
+        float* P = partial + (size_t)blockIdx.x * kNrcParams;
+        for (int L = warp >> 2; L < 6; L += 2 * kTrGroups) {
+            if (L < 5) {
+                uint32_t r[64];
+                const uint32_t col = tmem + 64u * (uint32_t)L + lanes;
+                AQ_TC_LD16(col + 0u, (r + 0));
+                AQ_TC_LD16(col + 16u, (r + 16));
+                AQ_TC_LD16(col + 32u, (r + 32));
+                AQ_TC_LD16(col + 48u, (r + 48));
+                tc_wait_ld();
+                float4* dst = reinterpret_cast<float4*>(P + (size_t)L * 4096 + (size_t)orow * 64);
+#pragma unroll
+                for (int c = 0; c < 16; ++c)
+                    dst[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
+                                         __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
+            } else {
+                uint32_t r[16];
+                AQ_TC_LD16(tmem + kTrW6Col + lanes, r);
+                tc_wait_ld();
+                for (int c = 0; c < kNrcOut; ++c) P[5 * 4096 + c * 64 + orow] = __uint_as_float(r[c]);
+            }
+        }
     }
+    if (tid == 0) {
+        double sum = 0.0;
+        for (int k = 0; k < 8 * kTrGroups; ++k) sum += (double)s_loss[k];
+        loss[blockIdx.x] = sum;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_slot), "r"(512u) : "memory");
 }
 
 // ---------------------------------------------------------------- host side
 size_t nrc_tc_weight_bytes() { return (size_t)kTcWeightBytes; }
 
-void nrc_pack_tc(aqua_ctx* ctx, const float* w, const float* inf, void* img_w, void* img_inf, void* img_bwd) {
+void nrc_pack_tc(aqua_ctx* ctx, const float* w, const float* inf, void* img_w, void* img_inf) {
     AQ_CUDA(cudaMemsetAsync(img_w, 0, kTcWeightBytes, ctx->stream));
     AQ_CUDA(cudaMemsetAsync(img_inf, 0, kTcWeightBytes, ctx->stream));
-    AQ_CUDA(cudaMemsetAsync(img_bwd, 0, kTcBwdBytes, ctx->stream));
-    k_nrc_pack_tc<<<(kNrcParams + 255) / 256, 256, 0, ctx->stream>>>(w, inf, (uint8_t*)img_w, (uint8_t*)img_inf,
-                                                                     (uint8_t*)img_bwd);
+    k_nrc_pack_tc<<<(kNrcParams + 255) / 256, 256, 0, ctx->stream>>>(w, inf, (uint8_t*)img_w, (uint8_t*)img_inf);
     AQ_CUDA(cudaGetLastError());
 }
 
@@ -572,9 +821,8 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n, float* out, uint32_t* err,
-                        uint32_t* acts, double* loss_zero) {
-    if (n <= 0) return;
+// n rows of 64 bf16 as boxes of 8 columns x 128 rows (zero past n).
+static CUtensorMap row_map(const uint16_t* X, int n) {
     if (((uintptr_t)X & 15) != 0) throw Error(AQUA_ERR_INVALID_ARG, "x must be 16-byte aligned");
     CUtensorMap map;
     const cuuint64_t dims[2] = {64, (cuuint64_t)n};
@@ -584,7 +832,13 @@ void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n
     CUresult r = tensor_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(X), dims,
                                       strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error(AQUA_ERR_CUDA, "cuTensorMapEncodeTiled failed for the query rows");
+    if (r != CUDA_SUCCESS) throw Error(AQUA_ERR_CUDA, "cuTensorMapEncodeTiled failed for the network's rows");
+    return map;
+}
+
+void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n, float* out, uint32_t* err) {
+    if (n <= 0) return;
+    const CUtensorMap map = row_map(X, n);
     if (!ctx->nrc_tc_ready) {  // once per context (one device)
         AQ_CUDA(cudaFuncSetAttribute(k_nrc_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcFwdSmemBytes));
         ctx->nrc_tc_ready = true;
@@ -592,233 +846,28 @@ void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n
     const int tiles = (n + kTcRows - 1) / kTcRows;
     const int grid = std::max(1, std::min(tiles, ctx->num_sms));
     launch_chained(k_nrc_forward_tc, dim3(grid), dim3(kTcFwdThreads), kTcFwdSmemBytes, ctx->stream, map, n,
-                   reinterpret_cast<const uint4*>(img), out, err, reinterpret_cast<uint4*>(acts), loss_zero);
+                   reinterpret_cast<const uint4*>(img), out, err);
     AQ_CUDA(cudaGetLastError());
 }
 
 
-// ---------------------------------------------------------------- weight gradients
-// dW_L = D_L^T x H_L over a chunk of rows (split-K, wgrad_chunk_rows; the Adam
-// kernel sums the chunk partials in order). Layer L of blockIdx.y: 0..4 ->
-// W1..W5 (H_0 = X, D = delta_{L+1}, 64 columns), 5 -> W6 (H_5, D = dY, 16
-// columns, 3 used). One tcgen05.mma per K = 16 rows: A = D^T (M = 128: the
-// 64 or 16 output features in rows 0.., zero rows above), B = H^T (N = 64
-// input features), both K-major with K = batch rows, accumulating in TMEM
-// (128 lanes x 64 FP32 columns). The 256 threads read each 128-row slice of
-// D and H with coalesced 16-byte loads (issued one slice ahead, into
-// registers), store it row-major to shared memory and transpose it there into
-// the no-swizzle core-matrix layout (8 batch rows of one feature = one
-// 16-byte core-matrix row); thread 0 issues the slice's MMAs and commits them
-// to an mbarrier, which the next slice's transpose waits for. The 84 KB of
-// shared memory let two CTAs share an SM. All waits are bounded.
-constexpr int kWgTcThreads = 256;
-constexpr int kWgTcChunk = 512;                 // rows per CTA (split-K chunk), at least
-constexpr int kWgTcMaxChunks = 64;              // larger batches get longer chunks
-constexpr int kWgTcSlice = 128;                 // rows per staged slice (MMA K = 8 x 16)
-constexpr int kWgTcABytes = 128 * kWgTcSlice * 2;  // A: 128 feature rows x 128 K
-constexpr int kWgTcBBytes = 64 * kWgTcSlice * 2;   // B: 64 feature rows x 128 K
-constexpr int kWgTcRawStride = 144;  // bytes per raw staged row: 128 + 16 (16-byte aligned; 8 rows start on 8 banks)
-constexpr int kWgTcRawBytes = kWgTcSlice * kWgTcRawStride;
-constexpr int kWgTcSmem = kWgTcABytes + kWgTcBBytes + 2 * kWgTcRawBytes + 1024;
-constexpr int kWgTcLoads = kWgTcSlice * 8 / kWgTcThreads;  // 16-byte loads per thread per matrix and slice
-static_assert(kWgTcChunk % kWgTcSlice == 0, "whole slices per chunk");
-static_assert(2 * kWgTcSmem <= 227 * 1024, "two CTAs per SM");
-// Rows per chunk for a batch of n rows: at least kWgTcChunk, and long enough
-// that at most kWgTcMaxChunks partials reach the Adam kernel, which sums
-// every parameter's partials in order (one thread per parameter).
-static int wgrad_chunk_rows(int n) {
-    const int per = (n + kWgTcMaxChunks - 1) / kWgTcMaxChunks;
-    return std::max(kWgTcChunk, (per + kWgTcChunk - 1) / kWgTcChunk * kWgTcChunk);
-}
-
-__global__ void __launch_bounds__(kWgTcThreads, 2) k_nrc_wgrad_tc(const uint16_t* __restrict__ X,
-                                                                  const uint16_t* __restrict__ acts,
-                                                                  const uint16_t* __restrict__ deltas,
-                                                                  const uint16_t* __restrict__ d6, int n,
-                                                                  int chunk_rows, float* __restrict__ partial,
-                                                                  uint32_t* __restrict__ err) {
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int L = blockIdx.y, ch = blockIdx.x;
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* sbase = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t sA = base, sB = base + (uint32_t)kWgTcABytes;
-    uint8_t* a = sbase;
-    uint8_t* bb = sbase + kWgTcABytes;
-    uint8_t* rawH = bb + kWgTcBBytes;
-    uint8_t* rawD = rawH + kWgTcRawBytes;
-    const int dcols = L == 5 ? 16 : 64;
-    const uint16_t* H = L == 0 ? X : acts + (size_t)(L - 1) * (size_t)n * 64;
-    const uint16_t* D = L == 5 ? d6 : deltas + (size_t)L * (size_t)n * 64;
-
-    // A's rows from dcols up stay zero for the whole chunk.
-    for (int i = tid; i < kWgTcABytes / 16; i += kWgTcThreads) reinterpret_cast<uint4*>(a)[i] = make_uint4(0, 0, 0, 0);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    grid_dep_wait();  // the activations and deltas come from the kernels before
-    grid_dep_launch();
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(64u)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc_idesc(128, 64);
-    const int row_begin = ch * chunk_rows;
-    const int slices = min(chunk_rows, n - row_begin + kWgTcSlice - 1) / kWgTcSlice;
-    // Raw row-major staging of one slice: H rows (128 B) and D rows (128 or
-    // 32 B), read with coalesced 16-byte loads into registers (zero past n).
-    const int dq = dcols / 8;  // 16-byte words per D row
-    uint4 rh[kWgTcLoads], rd[kWgTcLoads];
-    auto load_rows = [&](int r0) {
-#pragma unroll
-        for (int q = 0; q < kWgTcLoads; ++q) {
-            const int idx = tid + kWgTcThreads * q, row = r0 + (idx >> 3);
-            rh[q] = row < n ? __ldca(reinterpret_cast<const uint4*>(H + (size_t)row * 64) + (idx & 7)) : make_uint4(0, 0, 0, 0);
-            const int row_d = r0 + idx / dq;
-            rd[q] = (idx < kWgTcSlice * dq && row_d < n)
-                        ? __ldca(reinterpret_cast<const uint4*>(D + (size_t)row_d * dcols) + idx % dq)
-                        : make_uint4(0, 0, 0, 0);
-        }
-    };
-    auto store_raw = [&]() {
-#pragma unroll
-        for (int q = 0; q < kWgTcLoads; ++q) {
-            const int idx = tid + kWgTcThreads * q;
-            *reinterpret_cast<uint4*>(rawH + (size_t)(idx >> 3) * kWgTcRawStride + (size_t)(idx & 7) * 16) = rh[q];
-            if (idx < kWgTcSlice * dq)
-                *reinterpret_cast<uint4*>(rawD + (size_t)(idx / dq) * kWgTcRawStride + (size_t)(idx % dq) * 16) =
-                    rd[q];
-        }
-    };
-    load_rows(row_begin);
-    uint32_t par = 0;      // parity of the mbarrier's next completion
-    bool pending = false;  // the last slice's MMAs not yet waited for
-    bool ok = true;
-    for (int sl = 0; sl < slices; ++sl) {
-        // The slice's rows (prefetched) go to the raw buffers as they are;
-        // the next slice's rows are requested before this one is transposed.
-        store_raw();
-        if (sl + 1 < slices) load_rows(row_begin + (sl + 1) * kWgTcSlice);
-        // The previous slice's MMAs must have read A and B before the
-        // transpose overwrites them.
-        bool w = true;
-        if (pending && tid == 0) w = mbar_wait(smem_u32(&bar), par);
-        ok = __syncthreads_and(w) != 0;  // also: the raw buffers are complete
-        if (!ok) break;  // still pending: the drain below waits for it
-        if (pending) {
-            par ^= 1u;
-            pending = false;
-        }
-        // Transpose: feature f of rows 8j..8j+7 -> one 16-byte core-matrix row.
-        for (int it = tid; it < (64 + dcols) * 16; it += kWgTcThreads) {
-            const bool isA = it >= 64 * 16;
-            const int k = isA ? it - 64 * 16 : it;
-            const int cols = isA ? dcols : 64;
-            const int f = k % cols, j = k / cols;  // consecutive threads: consecutive features
-            const uint8_t* src = (isA ? rawD : rawH) + (size_t)(8 * j) * kWgTcRawStride + (size_t)f * 2;
-            uint32_t v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                v[q] = (uint32_t)*reinterpret_cast<const uint16_t*>(src + (size_t)(2 * q) * kWgTcRawStride) |
-                       ((uint32_t)*reinterpret_cast<const uint16_t*>(src + (size_t)(2 * q + 1) * kWgTcRawStride)
-                        << 16);
-            const int R = isA ? 128 : 64;
-            *reinterpret_cast<uint4*>((isA ? a : bb) + (size_t)j * R * 16 + (size_t)f * 16) =
-                make_uint4(v[0], v[1], v[2], v[3]);
-        }
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();  // the transpose is complete (and the raw buffers free)
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < kWgTcSlice / 16; ++k)
-                tc_mma(tmem, tc_desc(sA + (uint32_t)k * 2u * (128 * 16), 128 * 16),
-                       tc_desc(sB + (uint32_t)k * 2u * (64 * 16), 64 * 16), idesc, (sl > 0 || k > 0) ? 1u : 0u);
-            tc_commit(smem_u32(&bar));
-        }
-        pending = true;
-    }
-    // Drain: wait (bounded) for the commit still pending, so no MMA runs when
-    // the accumulator is read or the TMEM is freed.
-    if (pending) {
-        bool w = tid == 0 ? mbar_wait(smem_u32(&bar), par) : true;
-        ok = (__syncthreads_and(w) != 0) && ok;
-    }
-    tc_fence_after();
-    if (ok) {
-        // Lanes 0..63 hold rows (output features) 0..63; warps 0 and 1 read them.
-        const int orow = warp * 32 + lane;
-        if (warp < 2) {
-            uint32_t r[64];
-            const uint32_t lanes = (uint32_t)(warp * 32) << 16;
-            AQ_TC_LD16(tmem + lanes + 0u, (r + 0));
-            AQ_TC_LD16(tmem + lanes + 16u, (r + 16));
-            AQ_TC_LD16(tmem + lanes + 32u, (r + 32));
-            AQ_TC_LD16(tmem + lanes + 48u, (r + 48));
-            tc_wait_ld();
-            const int mrows = L == 5 ? kNrcOut : 64;
-            if (orow < mrows) {
-                float4* P = reinterpret_cast<float4*>(partial + (size_t)ch * kNrcParams + (size_t)L * 4096 +
-                                                      (size_t)orow * 64);
-#pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    P[c] = make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]),
-                                       __uint_as_float(r[4 * c + 2]), __uint_as_float(r[4 * c + 3]));
-            }
-        }
-    } else if (tid == 0) {
-        atomicExch(err, 1u);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(64u) : "memory");
-    }
-}
-
-int nrc_wgrad_tc_dev(aqua_ctx* ctx, const uint16_t* X, const uint32_t* acts, const uint32_t* deltas,
-                     const uint32_t* d6, int n, float* partial, uint32_t* err) {
+// One training step's gradients: per-CTA partials (kNrcParams each) and loss
+// sums for the Adam kernel; returns how many.
+int nrc_train_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, const float* T, int n, float inv_count,
+                     float* partial, double* loss, uint32_t* err) {
     if (n <= 0) return 0;
-    if (!ctx->nrc_tc_wg_ready) {
-        AQ_CUDA(cudaFuncSetAttribute(k_nrc_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgTcSmem));
-        ctx->nrc_tc_wg_ready = true;
+    const CUtensorMap map = row_map(X, n);
+    if (!ctx->nrc_tc_train_ready) {
+        AQ_CUDA(cudaFuncSetAttribute(k_nrc_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmemBytes));
+        ctx->nrc_tc_train_ready = true;
     }
-    const int rows = wgrad_chunk_rows(n);
-    const int chunks = (n + rows - 1) / rows;
-    launch_chained(k_nrc_wgrad_tc, dim3(chunks, 6), dim3(kWgTcThreads), kWgTcSmem, ctx->stream, X,
-                   reinterpret_cast<const uint16_t*>(acts), reinterpret_cast<const uint16_t*>(deltas),
-                   reinterpret_cast<const uint16_t*>(d6), n, rows, partial, err);
+    const int grid = std::min(nrc_train_tc_max_partials(ctx), (n + kTcRows - 1) / kTcRows);
+    launch_chained(k_nrc_train_tc, dim3(grid), dim3(kTrThreads), kTrSmemBytes, ctx->stream, map, T, n, inv_count,
+                   reinterpret_cast<const uint4*>(img), partial, loss, err);
     AQ_CUDA(cudaGetLastError());
-    return chunks;
+    return grid;
 }
 
-size_t nrc_tc_bwd_bytes() { return (size_t)kTcBwdBytes; }
-
-void nrc_backward_tc_dev(aqua_ctx* ctx, const void* img, const float* Y, const float* T, int n, float inv_count,
-                         const uint32_t* acts, uint32_t* deltas, uint32_t* d6, double* loss, uint32_t* err) {
-    if (n <= 0) return;
-    if (!ctx->nrc_tc_bwd_ready) {
-        AQ_CUDA(cudaFuncSetAttribute(k_nrc_backward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kTcBwdSmemBytes));
-        ctx->nrc_tc_bwd_ready = true;
-    }
-    const int tiles = (n + kTcRows - 1) / kTcRows;
-    const int grid = std::max(1, std::min(tiles, ctx->num_sms));
-    launch_chained(k_nrc_backward_tc, dim3(grid), dim3(kTcThreads), kTcBwdSmemBytes, ctx->stream, Y, T, n,
-                   inv_count, reinterpret_cast<const uint4*>(img), reinterpret_cast<const uint4*>(acts),
-                   reinterpret_cast<uint4*>(deltas), reinterpret_cast<uint4*>(d6), loss, err);
-    AQ_CUDA(cudaGetLastError());
-}
+int nrc_train_tc_max_partials(const aqua_ctx* ctx) { return ctx->num_sms; }
 
 }  // namespace aq

@@ -1338,7 +1338,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
             size_t r0 = (size_t)sidx * (size_t)batch;
             int rows = (int)std::min<size_t>((size_t)batch, nrec - r0);
             nrc_train_step_dev(ctx, net, nw.t_x + 64 * r0, nw.t_target + 3 * r0, rows);
-            launches += net.forward_tc ? 4 : 6;
+            launches += net.forward_tc ? 2 : 6;
         }
         AQ_CUDA(cudaMemcpyAsync(&loss, net.loss, 8, cudaMemcpyDeviceToHost, st));
         // Aim the next frame's training-path fraction at the record budget.
