@@ -2,17 +2,19 @@
 // scenes, uneven resolutions and sample counts) in one persistent launch,
 // replayed from a captured CUDA graph.
 //
-// Every lane of the persistent kernel owns one pixel at a time and keeps one
-// path of it in flight: a path advances one bounce per loop iteration, and
-// when it ends the lane starts the pixel's next sample at once (path
-// regeneration), so lanes do not wait for the longest path of their warp.
-// When a pixel has all its samples the lane writes it and, together with
-// the other idle lanes of its warp, takes the next pixels from a global
-// counter; jobs are laid out shortest first (pixels x spp), so small jobs
-// complete early. Contributions are summed in the wavefront's order
-// (emission, then next-event estimation, bounce after bounce, sample after
-// sample), so a job's image matches aqua_render's. The lane that finishes a
-// job's last pixel stamps the device clock, giving per-job latencies.
+// Every lane of the persistent kernel owns one unit at a time, a run of a
+// pixel's samples (all of them in large batches), and keeps one path of it in
+// flight: when the path ends the lane starts the next sample (path
+// regeneration), and when the unit is done it takes the next one from a
+// global counter, together with the other waiting lanes of its warp; jobs are
+// laid out shortest first (pixels x spp), so small jobs complete early. A
+// lane traces the path's extension and shadow rays one at a time and keeps
+// its walk between rounds, so lanes whose ray is done shade while others walk
+// on. Contributions are summed in the wavefront's order (emission, then
+// next-event estimation, bounce after bounce, sample after sample; a split
+// pixel's runs in order), so a job's image matches aqua_render's. The lane that
+// finishes a job's last pixel stamps the device clock, giving per-job
+// latencies.
 //
 // Path semantics are those of the wavefront (render.cu): `Perspective`
 // camera (scenes/cbox.json:516-543), Lambert + GGX `Principled`
@@ -27,10 +29,6 @@
 #include "shading.cuh"
 
 namespace aq {
-
-// Idle lanes of a warp fetch new pixels together once this many are idle
-// (or all are).
-constexpr int kBatchRefill = 1;
 
 __device__ __forceinline__ unsigned long long device_clock_ns() {
     unsigned long long t;
@@ -112,7 +110,7 @@ __device__ __forceinline__ bool shade_hit(const DevScene& S, int max_depth, int 
     const int depth = P.depth;
     if (h.tri < 0) {
         v3 e = mk(S.env[0], S.env[1], S.env[2]);
-        if (e.x > 0.0f || e.y > 0.0f || e.z > 0.0f) sum = sum + thr * e;
+        if (e.x > 0.0f || e.y > 0.0f || e.z > 0.0f) sum = fma3(thr, e, sum);
         return false;
     }
     const float4* tw = S.tris + 3 * (size_t)h.tri;
@@ -133,7 +131,7 @@ __device__ __forceinline__ bool shade_hit(const DevScene& S, int max_depth, int 
                 float pl = L.e2.w * h.t * h.t / (L.e1.w * cos_l);
                 w = power_heuristic(P.pdf_b, pl);
             }
-            sum = sum + thr * f3(L.le) * w;
+            sum = fma3(thr * f3(L.le), mk(w, w, w), sum);
         }
     }
     if (depth >= max_depth) return false;
@@ -222,97 +220,198 @@ __device__ __forceinline__ bool shade_hit(const DevScene& S, int max_depth, int 
     return alive;
 }
 
+// Lanes that wait for shading or a new pixel do so together, once this many
+// do (or none walks): 16 and 31 measured 4% and 1% slower than 24.
+constexpr int kBatchWait = 24;
+
 // Persistent kernel over all jobs' pixels. counters[0] = next pixel of the
 // whole batch, counters[1 + j] = finished pixels of job j. clocks[0] = launch
 // time, clocks[1 + j] = completion time of job j.
-// 4 resident blocks of 256 (64 registers): the spilled path state costs less
-// than the latency the extra warps hide (measured on the 64-job batch: 48,
-// 64 and 80 registers and the compiler's own 107 compared).
+// A lane keeps its walk between rounds, so lanes whose ray is done shade and
+// take new rays while others still walk (a walk per loop iteration waited for
+// the longest of 32 rays: 10 of 32 lanes active). 3 resident blocks of 256 (80
+// registers): the walk's and the path's state spill less than at 64 registers
+// (4 blocks, 3% slower). Walk nodes (load_walk) for the large scenes of a
+// mixed batch were tried: two node formats in one loop cost more than they
+// save (42.5 against 35.7 ms on 20 views of four scenes).
 template <bool FULL, int NODES>
-__global__ void __launch_bounds__(256, 4) k_batch(const DevScene* __restrict__ scenes, const DevJob* __restrict__ jobs, int njobs,
-                        uint32_t total_pixels, uint32_t* __restrict__ counters,
+__global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ scenes, const DevJob* __restrict__ jobs, int njobs,
+                        uint32_t total_items, uint32_t* __restrict__ counters, uint32_t* __restrict__ done_units,
+                        float4* __restrict__ partials,
                         unsigned long long* __restrict__ clocks, unsigned long long* __restrict__ stats) {
     __shared__ float lut[256];
-    __shared__ uint32_t first_pixel[kMaxBatchJobs + 1];
+    __shared__ uint32_t first_item[kMaxBatchJobs + 1];
     fill_srgb_lut(lut);
-    for (int j = threadIdx.x; j < njobs; j += blockDim.x) first_pixel[j] = jobs[j].pixel_begin;
-    if (threadIdx.x == 0) first_pixel[njobs] = total_pixels;
+    for (int j = threadIdx.x; j < njobs; j += blockDim.x) first_item[j] = jobs[j].item_begin;
+    if (threadIdx.x == 0) first_item[njobs] = total_items;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&clocks[0], 0ull, device_clock_ns());
     __syncthreads();
     const unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     uint32_t n_ext = 0, n_sh = 0, n_paths = 0;
-    bool have = false, drained = false;
+    bool have = false, walking = false, drained = false;
     int job = 0;
-    uint32_t pixel = 0, sample = 0;
+    uint32_t pixel = 0, sample = 0, sample_end = 0;
     v3 sum = mk(0.0f, 0.0f, 0.0f);
     LanePath P;
+    P.shadow = false;
+    // The ray in flight.
+    RayPre rp;
+    RayShear sh;
+    TraceResult r;
+    int32_t stack[kStackSize];
+    int sp = 0;
+    int32_t node = kTraversalDone, leaf = 0;
+    r.t = 0.0f; r.u = 0.0f; r.v = 0.0f; r.tri = -1; r.id = 0;
     while (true) {
-        // Idle lanes take the next pixels of the batch together.
-        const unsigned idle = __ballot_sync(kFull, !have);
-        if (!drained && idle != 0u && (__popc(idle) >= kBatchRefill || idle == kFull)) {
-            const int leader = __ffs(idle) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(&counters[0], (uint32_t)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if ((uint64_t)base + (uint64_t)__popc(idle) >= (uint64_t)total_pixels) drained = true;
-            if (!have) {
-                const uint32_t item = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (item < total_pixels) {
-                    int lo = 0, hi = njobs - 1;
-                    while (lo < hi) {  // last job whose first pixel <= item
-                        int mid = (lo + hi + 1) >> 1;
-                        if (first_pixel[mid] <= item) lo = mid;
-                        else hi = mid - 1;
+        // Lanes without a ray: finished ones shade and go on, free ones take
+        // the next pixels of the batch; together, once enough of them wait.
+        const unsigned act = __ballot_sync(kFull, walking);
+        const unsigned wait = __ballot_sync(kFull, !walking && (have || !drained));
+        if (wait != 0u && (__popc(wait) >= kBatchWait || act == 0u)) {
+            bool fresh = false;
+            if (have && !walking) {
+                const DevJob& J = jobs[job];
+                bool alive;
+                if (P.shadow) {
+                    if (r.tri < 0) sum = sum + P.contrib;
+                    P.shadow = false;
+                    alive = P.alive;
+                } else {
+                    alive = shade_hit<FULL>(scenes[J.scene], J.max_depth, J.rr_depth, lut, r, P, sum);
+                    alive = alive || P.shadow;
+                }
+                if (!alive) {
+                    // The path ended: the unit's next sample, or the unit is done.
+                    if (++sample < sample_end) {
+                        fresh = true;
+                    } else {
+                        have = false;
+                        bool pixel_done = true;
+                        if (J.units > 1) {
+                            // The lane that finishes a pixel's last unit sums them in order.
+                            const uint32_t k = (sample_end - 1u) / J.unit_spp;
+                            float4* part = partials + J.part_begin + pixel;
+                            __stcg(part + (size_t)k * J.pixels, make_float4(sum.x, sum.y, sum.z, 0.0f));
+                            __threadfence();
+                            pixel_done = atomicAdd(&done_units[J.done_begin + pixel], 1u) + 1u == J.units;
+                            if (pixel_done) {
+                                __threadfence();
+                                sum = mk(0.0f, 0.0f, 0.0f);
+                                for (uint32_t q = 0; q < J.units; ++q) sum = sum + f3(__ldcg(part + (size_t)q * J.pixels));
+                            }
+                        }
+                        if (pixel_done) {
+                            n_paths += (uint32_t)J.spp;
+                            const float inv = 1.0f / (float)J.spp;
+                            J.out[3 * (size_t)pixel + 0] = sum.x * inv;
+                            J.out[3 * (size_t)pixel + 1] = sum.y * inv;
+                            J.out[3 * (size_t)pixel + 2] = sum.z * inv;
+                            // Count finished pixels per job (one atomic per job among the lanes
+                            // finishing now); the lane that completes a job stamps the clock.
+                            const unsigned same = __match_any_sync(__activemask(), job);
+                            if (lane == __ffs(same) - 1) {
+                                const uint32_t k = (uint32_t)__popc(same);
+                                if (atomicAdd(&counters[1 + job], k) + k == J.pixels)
+                                    clocks[1 + job] = device_clock_ns();
+                            }
+                        }
                     }
-                    job = lo;
-                    pixel = item - first_pixel[lo];
-                    sample = 0;
-                    sum = mk(0.0f, 0.0f, 0.0f);
-                    start_sample(jobs[job], pixel, 0, P);
-                    have = true;
                 }
             }
+            __syncwarp();
+            const unsigned idle = __ballot_sync(kFull, !have);
+            if (!drained && idle != 0u) {
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if (lane == leader) base = atomicAdd(&counters[0], (uint32_t)__popc(idle));
+                base = __shfl_sync(kFull, base, leader);
+                if ((uint64_t)base + (uint64_t)__popc(idle) >= (uint64_t)total_items) drained = true;
+                if (!have) {
+                    const uint32_t item = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
+                    if (item < total_items) {
+                        int lo = 0, hi = njobs - 1;
+                        while (lo < hi) {  // last job whose first item <= item
+                            int mid = (lo + hi + 1) >> 1;
+                            if (first_item[mid] <= item) lo = mid;
+                            else hi = mid - 1;
+                        }
+                        job = lo;
+                        const DevJob& J = jobs[lo];
+                        const uint32_t k = (item - first_item[lo]) / J.pixels;
+                        pixel = item - first_item[lo] - k * J.pixels;
+                        sample = k * J.unit_spp;
+                        sample_end = min(sample + J.unit_spp, (uint32_t)J.spp);
+                        sum = mk(0.0f, 0.0f, 0.0f);
+                        have = fresh = true;
+                    }
+                }
+            }
+            if (fresh) start_sample(jobs[job], pixel, sample, P);
+            if (have && !walking) {
+                // The pending shadow ray, else the extension ray.
+                const bool any = P.shadow;
+                if (any) ++n_sh;
+                else ++n_ext;
+                const v3 o = (FULL && any) ? P.so : P.o, d = any ? P.sdir : P.dir;
+                rp.o = o;
+                rp.invd = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+                rp.tmin = 0.0f;
+                rp.tmax = any ? P.stmax : INFINITY;
+                sh = make_shear(o, d);
+                r.t = rp.tmax; r.u = 0.0f; r.v = 0.0f; r.tri = -1; r.id = 0x7fffffff;
+                sp = 0;
+                node = 0;
+                leaf = 0;
+                walking = true;
+            }
         }
-        if (!__any_sync(kFull, have)) break;
-        if (!have) continue;
-        const DevJob& J = jobs[job];
-        const DevScene& S = scenes[J.scene];
-        // One ray per iteration, from one call site: the pending shadow ray,
-        // else the extension ray.
-        const bool any = P.shadow;
-        if (any) ++n_sh;
-        else ++n_ext;
-        const TraceResult h = traverse_fast<NODES>(S, (FULL && any) ? P.so : P.o, any ? P.sdir : P.dir, 0.0f,
-                                            any ? P.stmax : INFINITY, any);
-        bool alive;
-        if (any) {
-            if (h.tri < 0) sum = sum + P.contrib;
-            P.shadow = false;
-            alive = P.alive;
-        } else {
-            alive = shade_hit<FULL>(S, J.max_depth, J.rr_depth, lut, h, P, sum);
-            if (P.shadow) continue;
-        }
-        if (alive) continue;
-        // The path ended: the pixel's next sample, or the pixel is done.
-        if (++sample < (uint32_t)J.spp) {
-            start_sample(J, pixel, sample, P);
+        if (!__any_sync(kFull, walking)) {
+            if (!__any_sync(kFull, have || !drained)) break;
             continue;
         }
-        n_paths += (uint32_t)J.spp;
-        const float inv = 1.0f / (float)J.spp;
-        J.out[3 * (size_t)pixel + 0] = sum.x * inv;
-        J.out[3 * (size_t)pixel + 1] = sum.y * inv;
-        J.out[3 * (size_t)pixel + 2] = sum.z * inv;
-        have = false;
-        // Count finished pixels per job (one atomic per job among the lanes
-        // finishing now); the lane that completes a job stamps the clock.
-        const unsigned same = __match_any_sync(__activemask(), job);
-        if (lane == __ffs(same) - 1) {
-            const uint32_t k = (uint32_t)__popc(same);
-            if (atomicAdd(&counters[1 + job], k) + k == J.pixels) clocks[1 + job] = device_clock_ns();
+        if (!walking) continue;
+        // One round of the walk: inner nodes with postponed leaves, then the leaves.
+        const DevScene& S = scenes[jobs[job].scene];
+        while (node >= 0) {
+            node = push_ordered(load_children<NODES>(S, node, rp, r.t), stack, sp);
+            if (node < 0 && node != kTraversalDone && leaf == 0) {
+                leaf = node;
+                node = sp > 0 ? stack[--sp] : kTraversalDone;
+            }
+            if (!__any_sync(__activemask(), leaf == 0)) break;
         }
+        while (leaf < 0) {
+            const int32_t code = ~leaf, first = code >> 3, cnt = code & 7;
+            bool stop = false;
+            for (int k = 0; k < cnt; ++k) {
+                const float4* tp = S.tris + 3 * (size_t)(first + k);
+                const float4 a = ldg_(tp), b = ldg_(tp + 1), c = ldg_(tp + 2);
+                const TriHit h = intersect_tri(sh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), mk(c.x, c.y, c.z), rp.tmin,
+                                               rp.tmax);
+                if (h.hit) {
+                    const int32_t id = __float_as_int(a.w);
+                    if (P.shadow) {
+                        r.tri = first + k;
+                        stop = true;
+                        break;
+                    }
+                    if (h.t < r.t || (h.t == r.t && id < r.id)) {
+                        r.t = h.t; r.u = h.u; r.v = h.v; r.tri = first + k; r.id = id;
+                    }
+                }
+            }
+            leaf = 0;
+            if (stop) {
+                node = kTraversalDone;
+                break;
+            }
+            if (node < 0 && node != kTraversalDone) {
+                leaf = node;
+                node = sp > 0 ? stack[--sp] : kTraversalDone;
+            }
+        }
+        if (node == kTraversalDone) walking = false;
     }
     for (int o = 16; o > 0; o >>= 1) {
         n_ext += __shfl_down_sync(kFull, n_ext, o);
@@ -351,8 +450,44 @@ struct BatchResult {
     std::vector<unsigned long long> clocks;
 };
 
+// Splits the pixels' samples into units (DevJob) for about `lanes` lanes (the
+// GPU's at the default launch shape, so that an image's rounding does not
+// depend on the shape). A pixel's samples run one after another on one lane, so the last
+// pixels of a small batch kept a few lanes busy long after the others had
+// run dry (a 51 x 145 view of the interior at 43 spp took 19 ms alone); units
+// short enough that each lane takes kUnitsPerLane of them bound that tail
+// (four views of up to 128^2 at 6 spp 2.41 -> 0.81 ms, ten of up to 300^2 at 16
+// spp 7.56 -> 3.31, twenty of up to 512^2 at 48 spp 41.4 -> 35.7). A large
+// batch keeps whole pixels.
+// Returns the items; pixels and partial sums of the split jobs by reference.
+constexpr uint64_t kBatchLanes = 768;  // per SM
+constexpr uint64_t kUnitsPerLane = 64;  // 16, 32 and 128: within 4%
+
+static uint32_t split_jobs(std::vector<DevJob>& jobs, uint64_t lanes, bool split, uint32_t& split_pixels,
+                           uint32_t& parts) {
+    uint64_t paths = 0;
+    for (const DevJob& j : jobs) paths += (uint64_t)j.pixels * (uint64_t)j.spp;
+    const uint64_t run = std::max<uint64_t>(1, paths / (lanes * kUnitsPerLane));
+    uint32_t items = 0;
+    split_pixels = parts = 0;
+    for (DevJob& j : jobs) {
+        j.unit_spp = split && run < (uint64_t)j.spp ? (uint32_t)run : (uint32_t)j.spp;
+        j.units = ((uint32_t)j.spp + j.unit_spp - 1) / j.unit_spp;
+        j.item_begin = items;
+        j.part_begin = j.done_begin = 0;
+        if (j.units > 1) {
+            j.part_begin = parts;
+            j.done_begin = split_pixels;
+            parts += j.units * j.pixels;
+            split_pixels += j.pixels;
+        }
+        items += j.units * j.pixels;
+    }
+    return items;
+}
+
 static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::vector<DevScene>& scenes,
-                               uint32_t total_pixels, const aqua_tuning& tune) {
+                               const aqua_tuning& tune, bool split) {
     const size_t n = jobs.size();
     int block = tune.block_trace > 0 ? tune.block_trace : 128;
     if (block != 64 && block != 128 && block != 256) throw Error(AQUA_ERR_INVALID_ARG, "block size must be 64, 128 or 256");
@@ -370,62 +505,85 @@ static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::ve
     int grid = ctx->num_sms * per_sm;
     cudaStream_t st = ctx->stream;
     BatchGraph& g = ctx->batch;
+    uint32_t parts = 0, split_pixels = 0;
+    uint32_t items = split_jobs(jobs, (uint64_t)ctx->num_sms * kBatchLanes, split, split_pixels, parts);
     bool reuse = same_batch(g, jobs, scenes, block, grid) && tune.use_graph != 0;
+    if (!reuse && split && g.exec && tune.use_graph != 0) {
+        // The last batch may have had to run unsplit (below).
+        std::vector<DevJob> whole = jobs;
+        uint32_t a = 0, b = 0;
+        split_jobs(whole, 1, false, a, b);
+        reuse = same_batch(g, whole, scenes, block, grid);
+    }
     if (!reuse) {
         batch_release(ctx);
         size_t off = 0;
-        auto take = [&](size_t b) { size_t o = off; off = (off + b + 255) / 256 * 256; return o; };
-        size_t o_s = take(sizeof(DevScene) * scenes.size()), o_j = take(sizeof(DevJob) * n),
-               o_c = take(4 * (n + 1)), o_t = take(8 * (n + 1)), o_st = take(8 * 4);
-        dev_alloc(ctx, g.buf, off);
+        size_t o_s = 0, o_j = 0, o_c = 0, o_t = 0, o_st = 0, o_d = 0, o_p = 0;
+        auto lay_out = [&]() {
+            off = 0;
+            auto take = [&](size_t b) { size_t o = off; off = (off + b + 255) / 256 * 256; return o; };
+            o_s = take(sizeof(DevScene) * scenes.size());
+            o_j = take(sizeof(DevJob) * n);
+            o_c = take(4 * (n + 1));
+            o_t = take(8 * (n + 1));
+            o_st = take(8 * 4);
+            o_d = take(4 * (size_t)split_pixels);
+            o_p = take(16 * (size_t)parts);
+        };
+        lay_out();
+        try {
+            dev_alloc(ctx, g.buf, off);
+        } catch (const Error& e) {
+            if (e.status != AQUA_ERR_OOM || parts == 0) throw;
+            (void)cudaGetLastError();  // no room for the partial sums: whole pixels need none
+            items = split_jobs(jobs, 1, false, split_pixels, parts);
+            lay_out();
+            dev_alloc(ctx, g.buf, off);
+        }
         char* b = (char*)g.buf.ptr;
         g.d_scenes = (DevScene*)(b + o_s);
         g.d_jobs = (DevJob*)(b + o_j);
         g.d_counters = (uint32_t*)(b + o_c);
         g.d_clocks = (unsigned long long*)(b + o_t);
         g.d_stats = (unsigned long long*)(b + o_st);
+        g.d_done = (uint32_t*)(b + o_d);
+        g.d_partials = (float4*)(b + o_p);
         AQ_CUDA(cudaMemcpyAsync(g.d_scenes, scenes.data(), sizeof(DevScene) * scenes.size(), cudaMemcpyHostToDevice, st));
         AQ_CUDA(cudaMemcpyAsync(g.d_jobs, jobs.data(), sizeof(DevJob) * n, cudaMemcpyHostToDevice, st));
         g.jobs = jobs;
         g.scenes = scenes;
         g.block = block;
         g.grid = grid;
-        g.units = total_pixels;
-        // One launch of the whole batch: counter resets + the persistent kernel.
-        auto enqueue = [&](cudaStream_t s) {
-            AQ_CUDA(cudaMemsetAsync(g.d_counters, 0, 4 * (n + 1), s));
-            AQ_CUDA(cudaMemsetAsync(g.d_clocks, 0, 8 * (n + 1), s));
-            AQ_CUDA(cudaMemsetAsync(g.d_stats, 0, 8 * 4, s));
-            kernel<<<grid, block, 0, s>>>(g.d_scenes, g.d_jobs, (int)n, total_pixels, g.d_counters, g.d_clocks,
-                                           g.d_stats);
-            AQ_CUDA(cudaGetLastError());
-        };
-        if (tune.use_graph != 0) {
-            AQ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            try {
-                enqueue(st);
-            } catch (...) {
-                cudaGraph_t tmp;
-                cudaStreamEndCapture(st, &tmp);
-                if (tmp) cudaGraphDestroy(tmp);
-                throw;
-            }
-            AQ_CUDA(cudaStreamEndCapture(st, &g.graph));
-            AQ_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
+        g.items = items;
+        g.split_pixels = split_pixels;
+    }
+    // One launch of the whole batch: counter resets + the persistent kernel.
+    auto enqueue = [&](cudaStream_t s) {
+        AQ_CUDA(cudaMemsetAsync(g.d_counters, 0, 4 * (n + 1), s));
+        AQ_CUDA(cudaMemsetAsync(g.d_clocks, 0, 8 * (n + 1), s));
+        AQ_CUDA(cudaMemsetAsync(g.d_stats, 0, 8 * 4, s));
+        if (g.split_pixels) AQ_CUDA(cudaMemsetAsync(g.d_done, 0, 4 * (size_t)g.split_pixels, s));
+        kernel<<<grid, block, 0, s>>>(g.d_scenes, g.d_jobs, (int)n, g.items, g.d_counters, g.d_done, g.d_partials,
+                                       g.d_clocks, g.d_stats);
+        AQ_CUDA(cudaGetLastError());
+    };
+    if (!reuse && tune.use_graph != 0) {
+        AQ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        try {
+            enqueue(st);
+        } catch (...) {
+            cudaGraph_t tmp;
+            cudaStreamEndCapture(st, &tmp);
+            if (tmp) cudaGraphDestroy(tmp);
+            throw;
         }
+        AQ_CUDA(cudaStreamEndCapture(st, &g.graph));
+        AQ_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
     }
     EventPair ev;
     AQ_CUDA(cudaEventRecord(ev.e[0], st));
-    if (g.exec) {
-        AQ_CUDA(cudaGraphLaunch(g.exec, st));
-    } else {
-        AQ_CUDA(cudaMemsetAsync(g.d_counters, 0, 4 * (n + 1), st));
-        AQ_CUDA(cudaMemsetAsync(g.d_clocks, 0, 8 * (n + 1), st));
-        AQ_CUDA(cudaMemsetAsync(g.d_stats, 0, 8 * 4, st));
-        kernel<<<grid, block, 0, st>>>(g.d_scenes, g.d_jobs, (int)n, total_pixels, g.d_counters, g.d_clocks,
-                                        g.d_stats);
-        AQ_CUDA(cudaGetLastError());
-    }
+    if (g.exec) AQ_CUDA(cudaGraphLaunch(g.exec, st));
+    else enqueue(st);
     AQ_CUDA(cudaEventRecord(ev.e[1], st));
     std::vector<unsigned long long> clocks(n + 1);
     unsigned long long hs[4] = {0, 0, 0, 0};
@@ -449,7 +607,7 @@ void render_batch(aqua_ctx* ctx, const aqua_job* in, size_t n, const aqua_tuning
     std::vector<DevScene> scenes;
     std::map<const aqua_scene*, int> scene_index;
     std::vector<DevJob> jobs(n);
-    uint32_t total_pixels = 0;
+    uint64_t total_pixels = 0;
     for (size_t i = 0; i < n; ++i) {
         const aqua_job& j = in[i];
         if (!j.scene || !j.rgb_out) throw Error(AQUA_ERR_INVALID_ARG, "job " + std::to_string(i) + ": scene and rgb_out must be non-NULL");
@@ -494,12 +652,11 @@ void render_batch(aqua_ctx* ctx, const aqua_job* in, size_t n, const aqua_tuning
     for (size_t k = 0; k < n; ++k) {
         sorted[k] = jobs[order[k]];
         rank[order[k]] = k;
-        sorted[k].pixel_begin = total_pixels;
-        if ((uint64_t)total_pixels + sorted[k].pixels > 0xFFFFFF00ull)
+        if (total_pixels + sorted[k].pixels > 0xFFFFFF00ull)
             throw Error(AQUA_ERR_INVALID_ARG, "a batch holds at most 2^32 - 256 pixels");
         total_pixels += sorted[k].pixels;
     }
-    BatchResult r = launch_jobs(ctx, sorted, scenes, total_pixels, tune);
+    BatchResult r = launch_jobs(ctx, sorted, scenes, tune, true);
     if (stats) {
         stats->device_ms = r.ms;
         stats->paths = r.paths;
@@ -541,8 +698,9 @@ void render_persistent(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg&
     d.max_depth = cfg.max_depth;
     d.rr_depth = cfg.rr_depth;
     d.pixels = (uint32_t)pixels;
-    d.pixel_begin = 0;
-    BatchResult r = launch_jobs(ctx, jobs, scenes, (uint32_t)pixels, tune);
+    // Whole pixels: one image whose samples run side by side is the wavefront's
+    // case.
+    BatchResult r = launch_jobs(ctx, jobs, scenes, tune, false);
     if (!device_film) {
         AQ_CUDA(cudaMemcpyAsync(rgb_out, film, 12 * pixels, cudaMemcpyDeviceToHost, ctx->stream));
         AQ_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -378,74 +378,16 @@ __device__ __forceinline__ TraceResult traverse(const DevScene& S, v3 o, v3 d, f
     }
 }
 
-// Traversal with postponed leaves (Aila & Laine 2009, "Understanding the
-// Efficiency of Ray Traversal on GPUs"): a lane that reaches a leaf parks it
-// and keeps walking inner nodes until every lane of the warp still walking
-// holds a leaf (warp vote), then all test triangles together. Boxes, culling
-// and triangle tests are those of traverse(), so the result (the minimum
-// (t, scene index) over all triangles hit, or any hit) is identical; only
-// the order of visits, and thus the work counts, differ. `any` (stop at the
-// first hit) is a run-time flag, so a kernel that traces both kinds of ray
-// from one call site holds one inlined copy of the walk.
-template <int NODES>
-__device__ __forceinline__ TraceResult traverse_fast(const DevScene& S, v3 o, v3 d, float tmin, float tmax,
-                                                     bool any) {
-    RayPre rp;
-    rp.o = o;
-    rp.invd = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    rp.tmin = tmin;
-    rp.tmax = tmax;
-    RayShear sh = make_shear(o, d);
-    TraceResult r;
-    r.t = tmax; r.u = 0.0f; r.v = 0.0f; r.tri = -1; r.id = 0x7fffffff;
-    int32_t stack[kStackSize];
-    int sp = 0;
-    int32_t node = 0, leaf = 0;
-    while (true) {
-        while (node >= 0) {
-            node = push_ordered(load_children<NODES>(S, node, rp, r.t), stack, sp);
-            if (node < 0 && node != kTraversalDone && leaf == 0) {
-                leaf = node;
-                node = sp > 0 ? stack[--sp] : kTraversalDone;
-            }
-            if (!__any_sync(__activemask(), leaf == 0)) break;
-        }
-        while (leaf < 0) {
-            int32_t code = ~leaf;
-            int32_t first = code >> 3, cnt = code & 7;
-            for (int k = 0; k < cnt; ++k) {
-                const float4* tp = S.tris + 3 * (size_t)(first + k);
-                float4 a = ldg_(tp), b = ldg_(tp + 1), c = ldg_(tp + 2);
-                TriHit h = intersect_tri(sh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), mk(c.x, c.y, c.z), tmin, tmax);
-                if (h.hit) {
-                    int32_t id = __float_as_int(a.w);
-                    if (any) {
-                        r.t = h.t; r.tri = first + k; r.id = id;
-                        return r;
-                    }
-                    if (h.t < r.t || (h.t == r.t && id < r.id)) {
-                        r.t = h.t; r.u = h.u; r.v = h.v; r.tri = first + k; r.id = id;
-                    }
-                }
-            }
-            leaf = 0;
-            if (node < 0 && node != kTraversalDone) {
-                leaf = node;
-                node = sp > 0 ? stack[--sp] : kTraversalDone;
-            }
-        }
-        if (node == kTraversalDone) return r;
-    }
-}
-
 // Persistent traversal of a queue of n rays with ray replacement (Aila &
 // Laine 2009, sec. 4: "replacing terminated rays"): each lane holds its own
 // ray; once at least kRefillLanes lanes of the warp have finished theirs (or
 // all have), the idle lanes take the next rays from *cursor together (one
-// atomic per warp). Between refills every lane runs rounds of
-// traverse_fast: walk inner nodes with postponed leaves, then test the
-// parked leaves. Boxes, culling and triangle tests are those of traverse(),
-// so every ray's result is the one traverse_fast returns.
+// atomic per warp). Between refills every lane runs rounds with postponed
+// leaves (same paper): a lane that reaches a leaf parks it and keeps walking
+// inner nodes until the warp vote says the walking lanes hold one, then all
+// test triangles together. Boxes, culling and triangle tests are those of
+// traverse(), so the result (the minimum (t, scene index) over all triangles
+// hit, or any hit) is identical; only the order of visits differs.
 //   load(i, o, d, tmin, tmax) -> uint32_t tag: fetches ray i of the queue;
 //   done(tag, r): called once per ray, by the lanes finishing in the same
 //                 round together (warp collectives inside are allowed).
@@ -519,7 +461,7 @@ __device__ __forceinline__ void traverse_lanes(const DevScene& S, uint32_t n, ui
         }
         if (!__any_sync(kFull, have)) break;
         if (!have) continue;
-        // One round of traverse_fast.
+        // One round.
         while (node >= 0) {
             Children c = load_children<NODES>(S, node, rp, r.t);
             if constexpr (KIND == kQueueAny && NODES == kNodesWalk) {

@@ -171,7 +171,11 @@ struct DevJob {
     float* out;              // width * height * 3 floats
     uint64_t seed;
     int32_t scene, spp, max_depth, rr_depth;
-    uint32_t pixels, pixel_begin;    // pixels of the job, its first pixel in the batch
+    uint32_t pixels;         // pixels of the job
+    // A pixel's samples are split into `units` runs of unit_spp (the last one
+    // shorter); unit k of pixel p is work item item_begin + k * pixels + p. With
+    // more than one, the runs' sums go to partials[part_begin + k * pixels + p].
+    uint32_t item_begin, units, unit_spp, part_begin, done_begin;
 };
 
 // The last batch, kept so an identical batch replays its CUDA graph.
@@ -182,12 +186,14 @@ struct BatchGraph {
     DevScene* d_scenes = nullptr;
     DevJob* d_jobs = nullptr;
     uint32_t* d_counters = nullptr;
+    uint32_t* d_done = nullptr;      // finished units per pixel of the split jobs
+    float4* d_partials = nullptr;
     unsigned long long* d_clocks = nullptr;
     unsigned long long* d_stats = nullptr;
     std::vector<DevJob> jobs;
     std::vector<DevScene> scenes;
     int block = 0, grid = 0;
-    uint32_t units = 0;
+    uint32_t items = 0, split_pixels = 0;
 };
 
 enum { kCntQ0 = 0, kCntQ1 = 1, kCntShadow = 2, kCntBucket0 = 10 };

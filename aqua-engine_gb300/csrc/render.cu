@@ -186,13 +186,11 @@ __device__ __forceinline__ uint32_t block_append(uint32_t* ctr, bool pred, uint3
     return k;
 }
 
-// *sum += a * b, one rounding per channel: spelled out, so that every variant
-// of the shading kernel rounds alike (the compiler may fuse a product into
-// the addition in one variant and not in another).
+// *sum += a * b (fma3).
 __device__ __forceinline__ void add_product(float4* sum, v3 a, v3 b) {
-    float4 f = *sum;
-    f.x = fmaf(a.x, b.x, f.x); f.y = fmaf(a.y, b.y, f.y); f.z = fmaf(a.z, b.z, f.z);
-    *sum = f;
+    const float4 f = *sum;
+    const v3 r = fma3(a, b, f3(f));
+    *sum = make_float4(r.x, r.y, r.z, f.w);
 }
 
 __device__ __forceinline__ void film_add(float4* film, uint32_t pixel, v3 c) {

@@ -10,6 +10,11 @@ namespace aq {
 
 __device__ __forceinline__ v3 f3(float4 a) { return mk(a.x, a.y, a.z); }
 
+// a * b + c, one rounding per channel. Emission is added this way wherever
+// radiance is summed: spelled out, so that every kernel rounds alike (the
+// compiler may fuse a product into the addition in one and not in another).
+__device__ __forceinline__ v3 fma3(v3 a, v3 b, v3 c) { return mk(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z)); }
+
 // Shirley-Chiu concentric square-to-disk mapping.
 __device__ __forceinline__ void concentric(float u, float v, float& x, float& y) {
     float a = 2.0f * u - 1.0f, b = 2.0f * v - 1.0f;
