@@ -9,15 +9,20 @@
 // tile in shared memory, and works through its tiles alone:
 //   - its first thread loads the next input tile with TMA (eight 128 x 8-column
 //     boxes) as soon as layer 1 has read the current one;
-//   - per layer the same thread issues four tcgen05.mma.kind::f16 (M = 128,
-//     N = 64, or 16 for the output layer, K = 16 each; BF16 x BF16 -> FP32)
-//     and commits them to the group's mbarrier. Layer 1 reads A from shared
-//     memory, layers 2-6 read it from TMEM;
+//   - per layer one of its warps, a different one in each group so that the
+//     four schedulers share the work, issues four tcgen05.mma.kind::f16 (M =
+//     128, N = 64, or 16 for the output layer, K = 16 each; BF16 x BF16 ->
+//     FP32) and commits them to the group's mbarrier. Layer 1 reads A from
+//     shared memory, layers 2-6 read it from TMEM;
 //   - each warp reads its 32 TMEM lanes (rows) of the accumulator with
 //     tcgen05.ld, applies ReLU, rounds to bf16 pairs and stores them back to
 //     the activation columns with tcgen05.st.
 // Activations never leave TMEM, and while one group is in its epilogue the
-// tensor core serves the others.
+// tensor core serves the others. Bound: the chain MMA -> epilogue -> MMA of six
+// layers, about 1000 cycles each with five tiles in flight. 16.8M rows: 774 us
+// when a single lane issued (110 cycles per MMA), 563 us issued by the
+// converged first warps, 536 us (31.3 G rows/s, 0.67 of the copy rate) spread
+// over the schedulers; 2.0M rows 107 -> 79 us.
 //
 // Shared-memory operands use the K-major layout without swizzle, with the
 // 8-row x 16-byte core matrices of one 8-column K slice stored back to back:
@@ -81,41 +86,58 @@ __global__ void k_nrc_pack_tc(const float* __restrict__ w, const float* __restri
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Shared-memory matrix descriptor: start address, leading byte offset (next
-// core matrix along K), stride byte offset (next 8 rows), all >> 4; bit 46 =
-// descriptor version 1; swizzle none.
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
-}
-
 // Instruction descriptor, kind::f16: D = F32 (bits 4-5), A = B = BF16 (bits
 // 7-9, 10-12), both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t tc_idesc(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+// Descriptors from a shared address >> 4 (no swizzle). K-major: `lbo` bytes
+// between groups of 8 along K, 128 between groups of 8 rows of the result.
+// MN-major: 128 between groups of 8 along K, `sbo` between groups of 8 rows.
+__device__ __forceinline__ uint64_t desc_k(uint32_t a, uint32_t lbo) {
+    return (uint64_t)(a | ((lbo >> 4) << 16)) | ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
+}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t a, uint32_t sbo) {
+    return (uint64_t)(a | ((128u >> 4) << 16)) | ((uint64_t)((sbo >> 4) | (1u << 14)) << 32);
 }
 
-// Same with A (128 rows x 16 bf16, two per 32-bit column) read from TMEM.
-__device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
+// True in one lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
+// tc_mma by the elected lane of a warp that runs converged.
+__device__ __forceinline__ void tc_issue(bool lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
         "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate));
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead));
+}
+// Same with A (128 rows x 16 bf16, two per 32-bit column) read from TMEM.
+__device__ __forceinline__ void tc_issue_ts(bool lead, uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead));
 }
 
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
@@ -215,11 +237,11 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
     __shared__ __align__(8) uint64_t bar_in[kTcFwdGroups], bar_mma[kTcFwdGroups];
     __shared__ uint32_t tmem_base_slot;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be uniform
     const int g = warp >> 2, q = warp & 3, gt = tid & 127;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* sbase = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t sW = base;
     const uint32_t sI = base + kTcWeightBytes + (uint32_t)g * kTcTileBytes;  // this group's input tile
 
     grid_dep_wait();  // the weights and inputs come from the kernels before
@@ -245,8 +267,10 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
     __syncthreads();
     tc_fence_after();
 
-    const uint32_t tmem = tmem_base_slot + (uint32_t)g * 64u;                    // this group's accumulator
-    const uint32_t tact = tmem_base_slot + kTcFwdActBase + (uint32_t)g * 32u;   // and activations
+    // All 512 columns were allocated, so they start at 0; with a constant the
+    // MMAs' TMEM addresses stay in uniform registers.
+    const uint32_t tmem = (uint32_t)g * 64u;                    // this group's accumulator
+    const uint32_t tact = kTcFwdActBase + (uint32_t)g * 32u;   // and activations
     const uint32_t lanes = (uint32_t)(q * 32) << 16;                             // this warp's lanes
     const uint32_t mb_in = smem_u32(&bar_in[g]), mb_mma = smem_u32(&bar_mma[g]);
     const int bar_id = 1 + g;
@@ -256,6 +280,7 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
     uint32_t ph_in = 0, ph_mma = 0;      // parity of the next phase to wait for
     uint32_t tma_par = 0, mma_par = 0;   // parity the work in flight will complete
     bool fail = false, tma_pending = false, mma_pending = false;
+    const bool lead = q == (g & 3) && elect_one();
 
     // Tiles interleave across CTAs first, so a small batch still spreads
     // over many SMs.
@@ -274,34 +299,33 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
         ph_in ^= 1u;
         if (group_any(bar_id, !ok)) { fail = true; break; }
         const int next = tile + stride;
+#pragma unroll
         for (int l = 0; l < 6; ++l) {
             const bool last = l == 5;
-            if (gt == 0) {
+            if (q == (g & 3)) {
+                // One of the group's warps issues, converged and with uniform
+                // operands (a single lane's code moves them to uniform
+                // registers for every MMA): K = 64 as four K = 16 steps, two
+                // core matrices of B each, and of A two core matrices (layer
+                // 1) or eight TMEM columns.
                 tc_fence_after();
                 const uint32_t idesc = tc_idesc(kTcRows, last ? kTcOutRows : 64);
-                const uint32_t b0 = sW + (uint32_t)l * kTcLayerBytes;
                 const uint32_t blbo = (last ? kTcOutRows : 64) * 16;
-                // K = 64 as four K = 16 steps: two core matrices of B each, and
-                // of A two core matrices (layer 1) or eight TMEM columns.
-                if (l == 0) {
+                const uint32_t b0 = (base >> 4) + (uint32_t)l * (kTcLayerBytes / 16);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma(tmem, tc_desc(sI + (uint32_t)k * 2u * (kTcRows * 16), kTcRows * 16),
-                               tc_desc(b0 + (uint32_t)k * 2u * blbo, blbo), idesc, k > 0 ? 1u : 0u);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        tc_mma_ts(tmem, tact + (uint32_t)k * 8u, tc_desc(b0 + (uint32_t)k * 2u * blbo, blbo), idesc,
-                                  k > 0 ? 1u : 0u);
+                for (uint32_t k = 0; k < 4; ++k) {
+                    const uint64_t bd = desc_k(b0 + k * 2u * (blbo / 16), blbo);
+                    if (l == 0) tc_issue(lead, tmem, desc_k((sI >> 4) + k * 256u, kTcRows * 16), bd, idesc, k > 0);
+                    else tc_issue_ts(lead, tmem, tact + k * 8u, bd, idesc, k > 0);
                 }
-                tc_commit(mb_mma);
+                if (lead) tc_commit(mb_mma);
                 mma_pending = true;
                 mma_par = ph_mma;
             }
             ok = mbar_wait(mb_mma, ph_mma);
             ph_mma ^= 1u;
             ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
-            if (gt == 0 && ok) mma_pending = false;
+            if (ok) mma_pending = false;
             // The input tile is free once layer 1 has read it: fetch the next one.
             if (l == 0 && gt == 0 && ok && next < tiles) {
                 tma_load_tile(&xmap, sI, mb_in, next * kTcRows);
@@ -340,11 +364,11 @@ __global__ void __launch_bounds__(kTcFwdThreads, 1)
         if (fail) break;
         tile = next;
     }
-    if (fail && gt == 0) {
-        atomicExch(err, 1u);
+    if (fail) {
         // Let what this group still has in flight land (bounded) before TMEM is freed.
-        if (mma_pending) mbar_wait(mb_mma, mma_par);
-        if (tma_pending) mbar_wait(mb_in, tma_par);
+        if (gt == 0) atomicExch(err, 1u);
+        if (lead && mma_pending) mbar_wait(mb_mma, mma_par);
+        if (gt == 0 && tma_pending) mbar_wait(mb_in, tma_par);
     }
     tc_fence_before();
     __syncthreads();
@@ -428,41 +452,6 @@ __device__ __forceinline__ uint32_t positive2(uint32_t h) {
     return __hgt2_mask(a, __floats2bfloat162_rn(0.0f, 0.0f));
 }
 
-// Descriptors from a shared address >> 4 (no swizzle). K-major: `lbo` bytes
-// between groups of 8 along K, 128 between groups of 8 rows of the result.
-// MN-major: 128 between groups of 8 along K, `sbo` between groups of 8 rows.
-__device__ __forceinline__ uint64_t desc_k(uint32_t a, uint32_t lbo) {
-    return (uint64_t)(a | ((lbo >> 4) << 16)) | ((uint64_t)((128u >> 4) | (1u << 14)) << 32);
-}
-__device__ __forceinline__ uint64_t desc_mn(uint32_t a, uint32_t sbo) {
-    return (uint64_t)(a | ((128u >> 4) << 16)) | ((uint64_t)((sbo >> 4) | (1u << 14)) << 32);
-}
-
-// True in one lane of the (converged) warp.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "elect.sync _|p, 0xffffffff;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(p));
-    return p != 0;
-}
-
-// tc_mma by the elected lane of a warp that runs converged.
-__device__ __forceinline__ void tc_issue(bool lead, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "setp.ne.b32 q, %5, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"((uint32_t)lead));
-}
 constexpr uint32_t kIdescAMn = 1u << 15, kIdescBMn = 1u << 16;  // A, B are MN-major
 
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
