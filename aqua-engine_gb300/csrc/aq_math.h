@@ -465,30 +465,54 @@ AQ_HD float bsdf_pdf(const Bsdf& b, v3 wo, v3 wi) {
     }
     return (1.0f - b.p_spec) * pd + b.p_spec * ps;
 }
-// GGX visible-normal sample for wo (Heitz 2018).
-AQ_HD v3 ggx_vndf(float a, v3 wo, float u1, float u2) {
+// Sine and cosine of one angle. On the device one range reduction serves both;
+// the values are those of sinf and cosf (checked for every angle 2 pi u of a
+// 24-bit u).
+AQ_HD void sincos_(float x, float& s, float& c) {
+#if defined(__CUDA_ARCH__)
+    sincosf(x, &s, &c);
+#else
+    s = sinf(x);
+    c = cosf(x);
+#endif
+}
+// A point of the unit disk in polar form: radius, sine and cosine of its angle.
+struct Disk {
+    float r, sn, cs;
+};
+AQ_HD Disk disk_point(float u1, float u2) {
+    Disk d;
+    d.r = sqrtf(u1);
+    sincos_(2.0f * kPi * u2, d.sn, d.cs);
+    return d;
+}
+// GGX visible-normal sample for wo (Heitz 2018) from a point of the disk.
+AQ_HD v3 ggx_vndf(float a, v3 wo, Disk p) {
     v3 Vh = normalize(mk(a * wo.x, a * wo.y, wo.z));
     float lensq = Vh.x * Vh.x + Vh.y * Vh.y;
     v3 T1 = lensq > 0.0f ? mk(-Vh.y, Vh.x, 0.0f) * (1.0f / sqrtf(lensq)) : mk(1.0f, 0.0f, 0.0f);
     v3 T2 = cross(Vh, T1);
-    float r = sqrtf(u1);
-    float phi = 2.0f * kPi * u2;
-    float t1 = r * cosf(phi), t2 = r * sinf(phi);
+    float t1 = p.r * p.cs, t2 = p.r * p.sn;
     float s = 0.5f * (1.0f + Vh.z);
-    t2 = (1.0f - s) * sqrtf(fmaxf_(1.0f - t1 * t1, 0.0f)) + s * t2;
-    v3 Nh = T1 * t1 + T2 * t2 + Vh * sqrtf(fmaxf_(0.0f, 1.0f - t1 * t1 - t2 * t2));
+    // The sums of two products below spell out which one is fused, so that the
+    // sample does not depend on the code around the call.
+    t2 = fmaf(1.0f - s, sqrtf(fmaxf_(1.0f - t1 * t1, 0.0f)), mul_rn(s, t2));
+    const float w = sqrtf(fmaxf_(0.0f, 1.0f - t1 * t1 - t2 * t2));
+    v3 Nh = mk(fmaf(Vh.x, w, fmaf(T1.x, t1, mul_rn(T2.x, t2))), fmaf(Vh.y, w, fmaf(T1.y, t1, mul_rn(T2.y, t2))),
+               fmaf(Vh.z, w, fmaf(T1.z, t1, mul_rn(T2.z, t2))));
     return normalize(mk(a * Nh.x, a * Nh.y, fmaxf_(0.0f, Nh.z)));
 }
 // Returns the sampled local direction; wi.z <= 0 means "no valid sample".
+// The lobes share the disk point of (u1, u2): a warp whose lanes pick
+// different lobes computes it once.
 AQ_HD v3 bsdf_sample(const Bsdf& b, v3 wo, float ulobe, float u1, float u2) {
+    const Disk p = disk_point(u1, u2);
     if (ulobe < b.p_spec) {
-        v3 Ne = ggx_vndf(b.alpha, wo, u1, u2);
+        v3 Ne = ggx_vndf(b.alpha, wo, p);
         float d = dot(wo, Ne);
         return Ne * (2.0f * d) - wo;
     }
-    float r = sqrtf(u1);
-    float phi = 2.0f * kPi * u2;
-    return mk(r * cosf(phi), r * sinf(phi), sqrtf(fmaxf_(0.0f, 1.0f - u1)));
+    return mk(p.r * p.cs, p.r * p.sn, sqrtf(fmaxf_(0.0f, 1.0f - u1)));
 }
 
 // Half vector of refraction between wo (this side) and wi (the other side,
@@ -576,7 +600,7 @@ AQ_HD float bsdf_pdf_full(const Bsdf& b, v3 wo, v3 wi) {
 AQ_HD v3 bsdf_sample_full(const Bsdf& b, v3 wo, float ulobe, float u1, float u2) {
     const v3 none = mk(0.0f, 0.0f, 0.0f);
     if (ulobe < b.p_glass) {
-        v3 h = ggx_vndf(b.alpha, wo, u1, u2);
+        v3 h = ggx_vndf(b.alpha, wo, disk_point(u1, u2));
         float co = dot(wo, h);
         float F = fresnel_dielectric(co, b.eta);
         if (ulobe < b.p_glass * F) {
@@ -594,8 +618,9 @@ AQ_HD v3 bsdf_sample_full(const Bsdf& b, v3 wo, float ulobe, float u1, float u2)
         float c2 = (1.0f - powf(b.cc_a2, 1.0f - u1)) / (1.0f - b.cc_a2);
         float ch = sqrtf(fminf_(fmaxf_(c2, 0.0f), 1.0f));
         float sh = sqrtf(fmaxf_(0.0f, 1.0f - ch * ch));
-        float phi = 2.0f * kPi * u2;
-        v3 h = mk(sh * cosf(phi), sh * sinf(phi), ch);
+        float sn, cs;
+        sincos_(2.0f * kPi * u2, sn, cs);
+        v3 h = mk(sh * cs, sh * sn, ch);
         float d = dot(wo, h);
         if (d < 0.0f) { h = -h; d = -d; }
         v3 r = h * (2.0f * d) - wo;

@@ -164,54 +164,16 @@ __device__ __forceinline__ bool shade_hit(const DevScene& S, int max_depth, int 
 #pragma unroll
     for (int k = 0; k < kBounceDims; ++k) u[k] = draw(P.st, P.inc);
     if (S.n_lights > 0 && wol.z > 0.0f) {
-        DevLight L = S.lights[pick_light(S, u[0])];
-        int ty = __float_as_int(L.p0.w);
-        float pmf = L.e2.w;
-        v3 contrib = mk(0, 0, 0), wi;
-        float dist = 0.0f;
-        bool below = false;  // light sample on the far side (glass lobe)
-        if (ty == AQUA_LIGHT_POINT) {
-            v3 dl = f3(L.p0) - p;
-            float d2 = dot(dl, dl);
-            dist = sqrtf(d2);
-            wi = dl * (1.0f / dist);
-            float cs = dot(wi, ns), cg = dot(wi, ng);
-            below = FULL && B.wglass > 0.0f && cs < 0.0f && cg < 0.0f;
-            if (((cs > 0.0f && cg > 0.0f) || below) && d2 > 0.0f) {
-                v3 wil = mk(dot(wi, T), dot(wi, Bt), cs);
-                contrib = thr * bsdf_eval_t<FULL>(B, wol, wil) * f3(L.le) * ((FULL ? fabsf(cs) : cs) / (d2 * pmf));
-            }
-        } else {
-            v3 le1 = f3(L.e1), le2 = f3(L.e2), xl;
-            if (ty == AQUA_LIGHT_QUAD) {
-                xl = f3(L.p0) + le1 * u[1] + le2 * u[2];
-            } else {
-                float su = sqrtf(u[1]);
-                xl = f3(L.p0) + le1 * (su * (1.0f - u[2])) + le2 * (su * u[2]);
-            }
-            v3 nl = normalize(cross(le1, le2));
-            v3 dl = xl - p;
-            float d2 = dot(dl, dl);
-            dist = sqrtf(d2);
-            wi = dl * (1.0f / dist);
-            float cl = -dot(wi, nl), cs = dot(wi, ns), cg = dot(wi, ng);
-            below = FULL && B.wglass > 0.0f && cs < 0.0f && cg < 0.0f;
-            if (cl > 0.0f && ((cs > 0.0f && cg > 0.0f) || below) && d2 > 0.0f) {
-                v3 wil = mk(dot(wi, T), dot(wi, Bt), cs);
-                float pl = pmf * d2 / (L.e1.w * cl);
-                float pb = bsdf_pdf_t<FULL>(B, wol, wil);
-                float w = power_heuristic(pl, pb);
-                contrib = thr * bsdf_eval_t<FULL>(B, wol, wil) * f3(L.le) * ((FULL ? fabsf(cs) : cs) * w / pl);
-            }
-        }
+        const LightSample ls = sample_light<FULL>(S, B, thr, p, ns, ng, T, Bt, wol, u);
+        const v3 contrib = ls.contrib;
         if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
             // The shadow ray leaves from the offset point on the light's
             // side; the extension ray sets its own origin afterwards.
             P.shadow = true;
             P.o = offset_ray(p, ng);
-            if (FULL) P.so = offset_ray(p, below ? -ng : ng);
-            P.sdir = wi;
-            P.stmax = dist * (1.0f - 1e-4f);
+            if (FULL) P.so = offset_ray(p, ls.below ? -ng : ng);
+            P.sdir = ls.wi;
+            P.stmax = ls.dist * (1.0f - 1e-4f);
             P.contrib = contrib;
         }
     }

@@ -165,7 +165,9 @@ __device__ __forceinline__ bool start_path(const DevScene& S, const WaveParams& 
 
 // Block-aggregated append: every thread of the block calls it together;
 // threads with pred set get consecutive entries of *ctr, with one atomic per
-// block instead of one per warp. s_warp: (warps + 1) shared words.
+// block instead of one per warp. s_warp: (warps + 1) shared words, not those
+// of the block's previous call (a barrier lies between a call and the next but
+// one).
 __device__ __forceinline__ uint32_t block_append(uint32_t* ctr, bool pred, uint32_t* s_warp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const unsigned m = __ballot_sync(0xffffffffu, pred);
@@ -181,9 +183,7 @@ __device__ __forceinline__ uint32_t block_append(uint32_t* ctr, bool pred, uint3
         s_warp[nw] = acc ? atomicAdd(ctr, acc) : 0u;
     }
     __syncthreads();
-    const uint32_t k = s_warp[nw] + s_warp[warp] + (uint32_t)__popc(m & ((1u << lane) - 1u));
-    __syncthreads();  // s_warp is reused by the next call
-    return k;
+    return s_warp[nw] + s_warp[warp] + (uint32_t)__popc(m & ((1u << lane) - 1u));
 }
 
 // *sum += a * b (fma3).
@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
     }
     uint32_t* out_cnt = &W.counters[cnt_out];
     unsigned long long done_paths = 0;
-    __shared__ uint32_t s_warp[5];
+    __shared__ uint32_t s_warp[2][5];
+    uint32_t turn = 0;
     // The whole block iterates together (the out-queue append is per block).
     for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + threadIdx.x;
@@ -484,53 +485,13 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
                 for (int k = 0; k < kBounceDims; ++k) u[k] = queried ? 0.0f : draw(st, inc);
                 // Next-event estimation: one light, one point, one shadow ray.
                 if (!queried && S.n_lights > 0 && wol.z > 0.0f) {
-                    DevLight L = S.lights[pick_light(S, u[0])];
-                    int ty = __float_as_int(L.p0.w);
-                    float pmf = L.e2.w;
-                    v3 contrib = mk(0, 0, 0), wi;
-                    float dist = 0.0f;
-                    bool below = false;  // light sample on the far side (glass lobe)
-                    if (ty == AQUA_LIGHT_POINT) {
-                        v3 dl = f3(L.p0) - p;
-                        float d2 = dot(dl, dl);
-                        dist = sqrtf(d2);
-                        wi = dl * (1.0f / dist);
-                        float cs = dot(wi, ns), cg = dot(wi, ng);
-                        below = FULL && B.wglass > 0.0f && cs < 0.0f && cg < 0.0f;
-                        if (((cs > 0.0f && cg > 0.0f) || below) && d2 > 0.0f) {
-                            v3 wil = mk(dot(wi, T), dot(wi, Bt), cs);
-                            contrib = thr * bsdf_eval_t<FULL>(B, wol, wil) * f3(L.le) *
-                                      ((FULL ? fabsf(cs) : cs) / (d2 * pmf));
-                        }
-                    } else {
-                        v3 le1 = f3(L.e1), le2 = f3(L.e2), xl;
-                        if (ty == AQUA_LIGHT_QUAD) {
-                            xl = f3(L.p0) + le1 * u[1] + le2 * u[2];
-                        } else {
-                            float su = sqrtf(u[1]);
-                            xl = f3(L.p0) + le1 * (su * (1.0f - u[2])) + le2 * (su * u[2]);
-                        }
-                        v3 nl = normalize(cross(le1, le2));
-                        v3 dl = xl - p;
-                        float d2 = dot(dl, dl);
-                        dist = sqrtf(d2);
-                        wi = dl * (1.0f / dist);
-                        float cl = -dot(wi, nl), cs = dot(wi, ns), cg = dot(wi, ng);
-                        below = FULL && B.wglass > 0.0f && cs < 0.0f && cg < 0.0f;
-                        if (cl > 0.0f && ((cs > 0.0f && cg > 0.0f) || below) && d2 > 0.0f) {
-                            v3 wil = mk(dot(wi, T), dot(wi, Bt), cs);
-                            float pl = pmf * d2 / (L.e1.w * cl);
-                            float pb = bsdf_pdf_t<FULL>(B, wol, wil);
-                            float w = power_heuristic(pl, pb);
-                            contrib = thr * bsdf_eval_t<FULL>(B, wol, wil) * f3(L.le) *
-                                      ((FULL ? fabsf(cs) : cs) * w / pl);
-                        }
-                    }
+                    const LightSample ls = sample_light<FULL>(S, B, thr, p, ns, ng, T, Bt, wol, u);
+                    const v3 contrib = ls.contrib;
                     if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
                         uint32_t k = warp_append(&W.counters[cnt_sh], true);
-                        v3 so = offset_ray(p, below ? -ng : ng);
+                        v3 so = offset_ray(p, ls.below ? -ng : ng);
                         W.sh_o[k] = make_float4(so.x, so.y, so.z, __int_as_float((int)pixel));
-                        W.sh_d[k] = make_float4(wi.x, wi.y, wi.z, dist * (1.0f - 1e-4f));
+                        W.sh_d[k] = make_float4(ls.wi.x, ls.wi.y, ls.wi.z, ls.dist * (1.0f - 1e-4f));
                         // w: 0, or the training path's id + 1 (negated: its
                         // targets only, the bounce lies past max_depth)
                         const int tid = NRC && tag ? ((int)depth < P.max_depth ? (int)(train_id + 1u)
@@ -576,7 +537,8 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
             cont = start_path<NRC>(S, P, W, s, j + 1);
         }
         }
-        const uint32_t k = block_append(out_cnt, cont, s_warp);
+        const uint32_t k = block_append(out_cnt, cont, s_warp[turn]);
+        turn ^= 1u;
         if (cont) W.q_out[k] = s;
     }
     for (int o = 16; o > 0; o >>= 1) done_paths += __shfl_down_sync(0xffffffffu, done_paths, o);

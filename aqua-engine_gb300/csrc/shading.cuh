@@ -94,6 +94,53 @@ __device__ __forceinline__ int pick_light(const DevScene& S, float u) {
 }
 
 
+// Next-event estimation at shading point p: one light, one point on it. The
+// contribution is zero when the sample cannot reach p or the BSDF is zero.
+struct LightSample {
+    v3 contrib, wi;
+    float dist;
+    bool below;  // on the far side of the surface (glass lobe)
+};
+template <bool FULL>
+__device__ __forceinline__ LightSample sample_light(const DevScene& S, const Bsdf& B, v3 thr, v3 p, v3 ns, v3 ng,
+                                                    v3 T, v3 Bt, v3 wol, const float* u) {
+    LightSample s;
+    const DevLight L = S.lights[pick_light(S, u[0])];
+    const int ty = __float_as_int(L.p0.w);
+    const float pmf = L.e2.w;
+    const bool point = ty == AQUA_LIGHT_POINT;
+    const v3 le1 = f3(L.e1), le2 = f3(L.e2);
+    v3 xl = f3(L.p0);
+    if (ty == AQUA_LIGHT_QUAD) {
+        xl = f3(L.p0) + le1 * u[1] + le2 * u[2];
+    } else if (!point) {
+        float su = sqrtf(u[1]);
+        xl = f3(L.p0) + le1 * (su * (1.0f - u[2])) + le2 * (su * u[2]);
+    }
+    const v3 dl = xl - p;
+    const float d2 = dot(dl, dl);
+    s.dist = sqrtf(d2);
+    s.wi = dl * (1.0f / s.dist);
+    const float cs = dot(s.wi, ns), cg = dot(s.wi, ng);
+    const float cl = point ? 1.0f : -dot(s.wi, normalize(cross(le1, le2)));
+    s.below = FULL && B.wglass > 0.0f && cs < 0.0f && cg < 0.0f;
+    s.contrib = mk(0.0f, 0.0f, 0.0f);
+    if (cl > 0.0f && ((cs > 0.0f && cg > 0.0f) || s.below) && d2 > 0.0f) {
+        const v3 wil = mk(dot(s.wi, T), dot(s.wi, Bt), cs);
+        float scale;
+        if (point) {
+            scale = (FULL ? fabsf(cs) : cs) / (d2 * pmf);
+        } else {
+            const float pl = pmf * d2 / (L.e1.w * cl);
+            const float pb = bsdf_pdf_t<FULL>(B, wol, wil);
+            const float w = power_heuristic(pl, pb);
+            scale = (FULL ? fabsf(cs) : cs) * w / pl;
+        }
+        s.contrib = thr * bsdf_eval_t<FULL>(B, wol, wil) * f3(L.le) * scale;
+    }
+    return s;
+}
+
 // sRGB decode table (IEC 61966-2-1), filled per block in shared memory.
 __device__ __forceinline__ void fill_srgb_lut(float* lut) {
     for (int i = threadIdx.x; i < 256; i += blockDim.x) {
