@@ -57,7 +57,8 @@ __device__ __forceinline__ void start_sample(const DevJob& J, uint32_t pixel, ui
     P.st = path_rng_state(J.seed, pixel, sample);
     P.inc = pixel_inc(pixel);
     float u0 = draw(P.st, P.inc), u1 = draw(P.st, P.inc), u2 = draw(P.st, P.inc), u3 = draw(P.st, P.inc);
-    camera_ray(J.cam, pixel, u0, u1, u2, u3, P.o, P.dir);
+    const uint32_t w = (uint32_t)J.cam.width, py = pixel / w;
+    camera_ray(J.cam, pixel - py * w, py, u0, u1, u2, u3, P.o, P.dir);
     P.thr = mk(1.0f, 1.0f, 1.0f);
     P.pdf_b = 0.0f;
     P.depth = 0;

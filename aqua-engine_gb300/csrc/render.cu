@@ -30,6 +30,25 @@
 
 namespace aq {
 
+// Division of 32-bit numbers by a number fixed per render: with m =
+// floor(2^32 / d) the product's high word is the quotient or one less.
+struct FastDiv {
+    uint32_t d, m;
+    __host__ void set(uint32_t divisor) {
+        d = divisor;
+        m = divisor > 1 ? (uint32_t)(((uint64_t)1 << 32) / divisor) : 0xffffffffu;
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t x, uint32_t& rem) const {
+        uint32_t q = __umulhi(x, m);
+        rem = x - q * d;
+        if (rem >= d) {
+            ++q;
+            rem -= d;
+        }
+        return q;
+    }
+};
+
 struct WaveParams {
     uint64_t seed;
     int32_t spp, spp_offset, max_depth, rr_depth;
@@ -51,7 +70,8 @@ struct WaveParams {
     uint32_t replicas;
     // Row subset (row_step > 1): film pixel p is image pixel
     // (row_begin + (p / width) * row_step) * width + p % width.
-    uint32_t row_begin, row_step, width;
+    uint32_t row_begin, row_step;
+    FastDiv by_width, by_pixels, by_spp;
 };
 
 struct WavePtrs {
@@ -89,58 +109,54 @@ enum { kCntFetchTrace = 6, kCntFetchShadow = 7, kCntShadow1 = 8 };
 
 // ---------------------------------------------------------------- helpers
 
-__device__ __forceinline__ uint32_t slot_work(const WaveParams& P, uint32_t s) {
-    if (P.replicas > 1) {
-        uint32_t r = s / P.pixels;
-        return r < (uint32_t)P.spp ? ((uint32_t)P.spp - r + P.replicas - 1) / P.replicas : 0u;
-    }
-    if (s >= P.pixels) return 0;
-    uint32_t npix = (P.pixels - s + P.slots - 1) / P.slots;
-    return npix * (uint32_t)P.spp;
-}
-
-// Image pixel of film pixel p (they differ for row-subset renders); the
-// image pixel names the camera ray and the random-number stream.
-__device__ __forceinline__ uint32_t image_pixel(const WaveParams& P, uint32_t p) {
+// Image pixel (px, py) of film pixel p (they differ for row-subset renders);
+// its number names the random-number stream.
+__device__ __forceinline__ uint32_t image_pixel(const WaveParams& P, uint32_t p, uint32_t& px, uint32_t& py) {
+    py = P.by_width(p, px);
     if (P.row_step <= 1) return p;
-    uint32_t r = p / P.width;
-    return (P.row_begin + r * P.row_step) * P.width + (p - r * P.width);
+    py = P.row_begin + py * P.row_step;
+    return py * P.by_width.d + px;
+}
+__device__ __forceinline__ uint32_t image_pixel(const WaveParams& P, uint32_t p) {
+    uint32_t px, py;
+    return P.row_step <= 1 ? p : image_pixel(P, p, px, py);
 }
 
 // Pixel (the film pixel of the stream), sample index and film entry of
-// work item j of slot s.
+// work item j of slot s; valid is false past the slot's last item.
 struct PathId {
     uint32_t pixel, sample, film;
+    bool valid;
 };
 __device__ __forceinline__ PathId path_id(const WaveParams& P, uint32_t s, uint32_t j) {
     PathId id;
     if (P.replicas > 1) {
-        uint32_t r = s / P.pixels;
-        id.pixel = s - r * P.pixels;
-        id.sample = (uint32_t)P.spp_offset + r + j * P.replicas;
+        const uint32_t r = P.by_pixels(s, id.pixel), k = r + j * P.replicas;
+        id.sample = (uint32_t)P.spp_offset + k;
         id.film = s;
+        id.valid = k < (uint32_t)P.spp;
     } else {
-        id.pixel = s + (j / (uint32_t)P.spp) * P.slots;
-        id.sample = (uint32_t)P.spp_offset + j % (uint32_t)P.spp;
+        uint32_t k;
+        id.pixel = s + P.by_spp(j, k) * P.slots;
+        id.sample = (uint32_t)P.spp_offset + k;
         id.film = id.pixel;
+        id.valid = id.pixel < P.pixels;
     }
     return id;
 }
 
-
-// Starts work item j of slot s (pixel, sample), writing its camera ray. The
-// path state's last word is depth (bits 0..7) | (training path id + 1) << 8;
-// the id is 0 outside the cache mode.
+// Starts work item `pid` (item j of slot s, valid), writing its camera ray.
+// The path state's last word is depth (bits 0..7) | (training path id + 1) <<
+// 8; the id is 0 outside the cache mode.
 template <bool NRC = false>
-__device__ __forceinline__ bool start_path(const DevScene& S, const WaveParams& P, const WavePtrs& W,
-                                           uint32_t s, uint32_t j) {
-    if (j >= slot_work(P, s)) return false;
-    PathId pid = path_id(P, s, j);
-    uint32_t pixel = image_pixel(P, pid.pixel), sample = pid.sample;
+__device__ __forceinline__ void start_path(const DevScene& S, const WaveParams& P, const WavePtrs& W, uint32_t s,
+                                           uint32_t j, const PathId& pid) {
+    uint32_t px, py;
+    const uint32_t pixel = image_pixel(P, pid.pixel, px, py), sample = pid.sample;
     uint64_t st = path_rng_state(P.seed, pixel, sample), inc = pixel_inc(pixel);
     float u0 = draw(st, inc), u1 = draw(st, inc), u2 = draw(st, inc), u3 = draw(st, inc);
     v3 o, d;
-    camera_ray(S.cam, pixel, u0, u1, u2, u3, o, d);
+    camera_ray(S.cam, px, py, u0, u1, u2, u3, o, d);
     W.ray_o[s] = make_float4(o.x, o.y, o.z, 0.0f);
     W.ray_d[s] = make_float4(d.x, d.y, d.z, INFINITY);
     W.tp[s] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -160,7 +176,6 @@ __device__ __forceinline__ bool start_path(const DevScene& S, const WaveParams& 
         }
     }
     W.pst[s] = make_uint4((uint32_t)st, (uint32_t)(st >> 32), j, tag);
-    return true;
 }
 
 // Block-aggregated append: every thread of the block calls it together;
@@ -210,7 +225,7 @@ __global__ void k_raygen(DevScene S, WaveParams P, WavePtrs W) {
         W.counters[kCntShadow] = 0;
     }
     for (uint32_t s = tid; s < n; s += gridDim.x * blockDim.x) {
-        start_path<NRC>(S, P, W, s, 0);
+        start_path<NRC>(S, P, W, s, 0, path_id(P, s, 0));
         W.q_in[s] = s;
     }
 }
@@ -534,7 +549,11 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
         }
         if (!cont) {
             ++done_paths;
-            cont = start_path<NRC>(S, P, W, s, j + 1);
+            const PathId next = path_id(P, s, j + 1);
+            if (next.valid) {
+                start_path<NRC>(S, P, W, s, j + 1, next);
+                cont = true;
+            }
         }
         }
         const uint32_t k = block_append(out_cnt, cont, s_warp[turn]);
@@ -858,7 +877,7 @@ static size_t plan_rows(const aqua_integrator_cfg& cfg, const DevCamera& cam, Wa
     size_t rows = h;
     P.row_begin = 0;
     P.row_step = 1;
-    P.width = (uint32_t)w;
+    P.by_width.set((uint32_t)w);
     if (cfg.row_step > 1) {
         if (cfg.row_begin < 0 || cfg.row_begin >= cfg.row_step || (size_t)cfg.row_begin >= h)
             throw Error(AQUA_ERR_INVALID_ARG, "row_begin must lie in [0, row_step) and below the image height");
@@ -895,6 +914,8 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     P.rr_depth = cfg.rr_depth;
     P.slots = (uint32_t)slots;
     P.pixels = (uint32_t)pixels;
+    P.by_pixels.set(P.pixels);
+    P.by_spp.set((uint32_t)P.spp);
     P.nb = (uint32_t)nb;
     WavePtrs W;
     W.ray_o = w.ray_o; W.ray_d = w.ray_d; W.hit = w.hit; W.tp = w.tp; W.pst = w.pst;
@@ -1169,6 +1190,8 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     P.rr_depth = cfg.rr_depth;
     P.slots = (uint32_t)slots;
     P.pixels = (uint32_t)pixels;
+    P.by_pixels.set(P.pixels);
+    P.by_spp.set((uint32_t)P.spp);
     P.nb = (uint32_t)nb;
     P.query_depth = query_depth;
     P.spread_c = 0.01f;  // Mueller et al. 2021
@@ -1427,6 +1450,8 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
     P.rr_depth = cfg.rr_depth;
     P.slots = (uint32_t)slots;
     P.pixels = (uint32_t)pixels;
+    P.by_pixels.set(P.pixels);
+    P.by_spp.set((uint32_t)P.spp);
     P.nb = 0;  // unsorted shading: no per-material buckets
     WavePtrs W;
     size_t off = 0;

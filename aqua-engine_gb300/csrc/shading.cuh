@@ -26,9 +26,8 @@ __device__ __forceinline__ void concentric(float u, float v, float& x, float& y)
     y = r * sinf(phi);
 }
 
-__device__ __forceinline__ void camera_ray(const DevCamera& c, uint32_t pixel, float u0, float u1, float u2,
-                                           float u3, v3& o, v3& d) {
-    uint32_t px = pixel % (uint32_t)c.width, py = pixel / (uint32_t)c.width;
+__device__ __forceinline__ void camera_ray(const DevCamera& c, uint32_t px, uint32_t py, float u0, float u1,
+                                           float u2, float u3, v3& o, v3& d) {
     float sx = (2.0f * (((float)px + u0) / (float)c.width) - 1.0f) * c.tan_half * c.aspect;
     float sy = (1.0f - 2.0f * (((float)py + u1) / (float)c.height)) * c.tan_half;
     v3 dc = mk(sx, sy, -1.0f), oc = mk(0, 0, 0);
