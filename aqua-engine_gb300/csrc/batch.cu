@@ -460,11 +460,7 @@ static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::ve
     for (const DevScene& sc : scenes) qbvh = qbvh || sc.qbvh != 0;
     auto kernel = full ? (qbvh ? k_batch<true, kNodesOwn> : k_batch<true, kNodesFull>)
                        : (qbvh ? k_batch<false, kNodesOwn> : k_batch<false, kNodesFull>);
-    int per_sm = tune.blocks_per_sm;
-    if (per_sm <= 0) {
-        AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
-        per_sm = std::max(per_sm, 1);
-    }
+    const int per_sm = tune.blocks_per_sm > 0 ? tune.blocks_per_sm : resident_blocks(ctx, kernel, block);
     int grid = ctx->num_sms * per_sm;
     cudaStream_t st = ctx->stream;
     BatchGraph& g = ctx->batch;
@@ -543,13 +539,13 @@ static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::ve
         AQ_CUDA(cudaStreamEndCapture(st, &g.graph));
         AQ_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
     }
-    EventPair ev;
+    EventPair& ev = timer(ctx);
     AQ_CUDA(cudaEventRecord(ev.e[0], st));
     if (g.exec) AQ_CUDA(cudaGraphLaunch(g.exec, st));
     else enqueue(st);
     AQ_CUDA(cudaEventRecord(ev.e[1], st));
     std::vector<unsigned long long> clocks(n + 1);
-    unsigned long long hs[4] = {0, 0, 0, 0};
+    unsigned long long* const hs = ctx->pinned_stats;
     AQ_CUDA(cudaMemcpyAsync(clocks.data(), g.d_clocks, 8 * (n + 1), cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaMemcpyAsync(hs, g.d_stats, 8 * 4, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));

@@ -332,7 +332,7 @@ AQUA_API aqua_status aqua_create(aqua_ctx** out, const aqua_options* opt) {
     cudaError_t e = cudaSetDevice(dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->pinned_counter, 64, cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->pinned_counter, 256, cudaHostAllocDefault);
     if (e != cudaSuccess) {
         g_create_error = std::string("CUDA initialisation failed: ") + cudaGetErrorString(e);
         cudaGetLastError();
@@ -340,6 +340,8 @@ AQUA_API aqua_status aqua_create(aqua_ctx** out, const aqua_options* opt) {
         delete ctx;
         return AQUA_ERR_CUDA;
     }
+    ctx->pinned_stats = reinterpret_cast<unsigned long long*>(ctx->pinned_counter + 16);
+    ctx->pinned_loss = reinterpret_cast<double*>(ctx->pinned_stats + 16);
     ctx->device = dev;
     ctx->verbose = opt ? opt->verbose : 0;
     ctx->fail_alloc_after = opt ? opt->fail_alloc_after : 0;
@@ -363,6 +365,7 @@ AQUA_API void aqua_destroy(aqua_ctx* ctx) {
     dev_free(ctx->persist_film);
     dev_free(ctx->trace_stats);
     for (auto e : ctx->events) cudaEventDestroy(e);
+    ctx->timer.reset();
     if (ctx->pinned_counter) cudaFreeHost(ctx->pinned_counter);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -902,15 +905,13 @@ AQUA_API aqua_status aqua_nrc_forward(aqua_ctx* ctx, aqua_nrc* n, const uint16_t
         } else {
             need(((uintptr_t)x & 15) == 0, "x must be 16-byte aligned");
         }
-        std::unique_ptr<EventPair> ev;
-        if (flags & AQUA_NRC_TIMING) {
-            ev.reset(new EventPair());
-            AQ_CUDA(cudaEventRecord(ev->e[0], ctx->stream));
-        }
+        EventPair* ev = flags & AQUA_NRC_TIMING ? &timer(ctx) : nullptr;
+        if (ev) AQ_CUDA(cudaEventRecord(ev->e[0], ctx->stream));
         nrc_forward_dev(ctx, n->net, d_x, (int)cnt, d_out);
         if (ev) AQ_CUDA(cudaEventRecord(ev->e[1], ctx->stream));
         if (!(flags & AQUA_NRC_DEVICE_PTRS))
             AQ_CUDA(cudaMemcpyAsync(out, d_out, 12 * cnt, cudaMemcpyDeviceToHost, ctx->stream));
+        nrc_read_back(ctx, n->net);
         AQ_CUDA(cudaStreamSynchronize(ctx->stream));
         nrc_check_tc(ctx, n->net);
         if (ev) n->last_ms = ev->ms();
@@ -955,22 +956,15 @@ AQUA_API aqua_status aqua_nrc_train_step(aqua_ctx* ctx, aqua_nrc* n, const uint1
         } else {
             need(((uintptr_t)x & 15) == 0, "x must be 16-byte aligned");
         }
-        std::unique_ptr<EventPair> ev;
-        if (flags & AQUA_NRC_TIMING) {
-            ev.reset(new EventPair());
-            AQ_CUDA(cudaEventRecord(ev->e[0], ctx->stream));
-        }
+        EventPair* ev = flags & AQUA_NRC_TIMING ? &timer(ctx) : nullptr;
+        if (ev) AQ_CUDA(cudaEventRecord(ev->e[0], ctx->stream));
         nrc_train_step_dev(ctx, n->net, d_x, d_t, (int)cnt);
         if (ev) AQ_CUDA(cudaEventRecord(ev->e[1], ctx->stream));
-        struct {
-            double loss;
-            uint32_t tc_err, pad;
-        } rb{};  // the loss and, right after it, the tcgen05 error flag
-        AQ_CUDA(cudaMemcpyAsync(&rb, n->net.loss, 16, cudaMemcpyDeviceToHost, ctx->stream));
+        nrc_read_back(ctx, n->net);
         AQ_CUDA(cudaStreamSynchronize(ctx->stream));
-        if (rb.tc_err) nrc_check_tc(ctx, n->net);  // resets the flag and throws
+        nrc_check_tc(ctx, n->net);
         if (ev) n->last_ms = ev->ms();
-        const double l = rb.loss;
+        const double l = *ctx->pinned_loss;
         if (loss) *loss = l / (double)(cnt * kNrcOut);
     });
 }

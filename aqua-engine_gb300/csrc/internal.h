@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <map>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -109,7 +111,8 @@ struct Workspace {
     float4* sh_c = nullptr;   // (contribution.rgb, 0)
     float4* film = nullptr;   // per-pixel sum
     uint32_t* counters = nullptr;   // see kCnt*
-    unsigned long long* stats = nullptr;  // see kStat*
+    unsigned long long* stats = nullptr;  // see kStat*; right behind the counters
+    size_t counter_bytes = 0;  // counters and statistics together
     float* out_rgb = nullptr;  // staging for host films (pixels * 3)
 };
 
@@ -233,7 +236,13 @@ struct aqua_ctx {
     aq::Workspace ws;
     aq::NrcWorkspace nrc_ws;
     aq::BatchGraph batch;
-    unsigned int* pinned_counter = nullptr;  // host-mapped copy of queue counts
+    // Page-locked words that calls read small results back into: a copy to
+    // pageable memory is staged by the driver and waits for it.
+    unsigned int* pinned_counter = nullptr;  // 16 queue counts
+    unsigned long long* pinned_stats = nullptr;  // 16 statistics
+    double* pinned_loss = nullptr;           // the training loss and, after it, the tcgen05 error flag
+    std::unique_ptr<aq::EventPair> timer;    // timing of one stretch of the stream, created on first use
+    std::map<std::pair<const void*, int>, int> resident;  // occupancy by kernel and block size
     std::vector<cudaEvent_t> events;         // pool for stage timing
     aq::DevBuf trace_rays, trace_hits;       // staging for host-pointer traces
     aq::DevBuf persist_film;                 // device film of host-film persistent renders
@@ -252,6 +261,23 @@ namespace aq {
 // 3.57 / 3.77 ms and 188 / 192 us; 33k 4.32 / 4.41 ms and 228 / 231 us; 131k
 // 4.82 / 4.87 ms and 260 / 252 us; the interior's 294k 47.9 / 40.8 ms.
 constexpr size_t kWalkNodesFrom = 150000;
+
+inline EventPair& timer(aqua_ctx* ctx) {
+    if (!ctx->timer) ctx->timer.reset(new EventPair());
+    return *ctx->timer;
+}
+
+// Blocks of the kernel that fit one SM, asked of the driver once per context.
+template <class K>
+int resident_blocks(aqua_ctx* ctx, K kernel, int block) {
+    int& n = ctx->resident[{(const void*)kernel, block}];
+    if (n == 0) {
+        int b = 0;
+        AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (const void*)kernel, block, 0));
+        n = b > 0 ? b : 1;
+    }
+    return n;
+}
 
 // Device allocation through the context (honours the fail_alloc_after hook).
 void dev_alloc(aqua_ctx* ctx, DevBuf& b, size_t bytes);
@@ -313,7 +339,10 @@ void nrc_forward_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, int n
 int nrc_train_tc_dev(aqua_ctx* ctx, const void* img, const uint16_t* X, const float* T, int n, float inv_count,
                      float* partial, double* loss, uint32_t* err);
 int nrc_train_tc_max_partials(const aqua_ctx* ctx);
-// Throws when a tcgen05 launch since the last check gave up waiting (syncs the stream).
+// Reads the last step's loss and the tcgen05 error flag back with the stream's
+// next synchronisation, after which nrc_check_tc throws when a tcgen05 launch
+// since the last check gave up waiting.
+void nrc_read_back(aqua_ctx* ctx, NrcNet& net);
 void nrc_check_tc(aqua_ctx* ctx, NrcNet& net);
 
 // Render on the library's fixed static scratch array; no device allocation.

@@ -566,15 +566,16 @@ void nrc_train_step_dev(aqua_ctx* ctx, NrcNet& net, const uint16_t* X, const flo
     net.launches += net.forward_tc ? 2 : 6;
 }
 
+void nrc_read_back(aqua_ctx* ctx, NrcNet& net) {
+    AQ_CUDA(cudaMemcpyAsync(ctx->pinned_loss, net.loss, 16, cudaMemcpyDeviceToHost, ctx->stream));
+}
+
 void nrc_check_tc(aqua_ctx* ctx, NrcNet& net) {
-    if (!net.forward_tc) return;
-    uint32_t e = 0;
-    AQ_CUDA(cudaMemcpyAsync(&e, net.tc_err, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    AQ_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (e) {
-        AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 4, ctx->stream));
-        throw Error(AQUA_ERR_TIMEOUT, "tensor-core inference: an MMA completion wait expired");
-    }
+    uint32_t e;
+    memcpy(&e, ctx->pinned_loss + 1, 4);
+    if (!net.forward_tc || !e) return;
+    AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 4, ctx->stream));
+    throw Error(AQUA_ERR_TIMEOUT, "tensor-core kernel: a completion wait expired");
 }
 
 void nrc_encode_dev(aqua_ctx* ctx, NrcNet& net, const float* raw, int n, uint16_t* X) {

@@ -729,6 +729,7 @@ static void ensure_workspace(aqua_ctx* ctx, size_t slots, size_t buckets, size_t
     w.film = (float4*)(b + o_film);
     w.counters = (uint32_t*)(b + o_cnt);
     w.stats = (unsigned long long*)(b + o_st);
+    w.counter_bytes = o_st + 8 * 16 - o_cnt;
     w.out_rgb = (float*)(b + o_out);
     w.slots = slots; w.buckets = buckets; w.pixels = pixels;
 }
@@ -776,11 +777,7 @@ static FusedKernel fused_kernel(int format) {
 
 template <class K>
 static int grid_for(aqua_ctx* ctx, K kernel, int block, int blocks_per_sm) {
-    int per_sm = blocks_per_sm;
-    if (per_sm <= 0) {
-        AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
-        per_sm = std::max(per_sm, 1);
-    }
+    const int per_sm = blocks_per_sm > 0 ? blocks_per_sm : resident_blocks(ctx, kernel, block);
     return ctx->num_sms * per_sm;
 }
 
@@ -946,8 +943,7 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     ev1 = tt.get();
 
     AQ_CUDA(cudaMemsetAsync(w.film, 0, 16 * pixels * plan.replicas, st));
-    AQ_CUDA(cudaMemsetAsync(w.stats, 0, 8 * 16, st));
-    AQ_CUDA(cudaMemsetAsync(w.counters, 0, 4 * (kCntBucket0 + std::max<size_t>(nb, 1)), st));
+    AQ_CUDA(cudaMemsetAsync(w.counters, 0, w.counter_bytes, st));  // and the statistics behind them
     AQ_CUDA(cudaEventRecord(ev0, st));
     uint64_t launches = 0;
     W.q_in = w.q[0];
@@ -1011,7 +1007,7 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     AQ_CUDA(cudaEventRecord(ev1, st));
     if (!(flags & AQUA_RENDER_DEVICE_FILM))
         AQ_CUDA(cudaMemcpyAsync(rgb_out, w.out_rgb, 12 * pixels, cudaMemcpyDeviceToHost, st));
-    unsigned long long hs[16];
+    unsigned long long* const hs = ctx->pinned_stats;
     AQ_CUDA(cudaMemcpyAsync(hs, w.stats, 8 * 16, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
     check_drained(hs[kStatPaths], pixels, cfg.spp);
@@ -1239,8 +1235,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     StageTimer tm{ctx, true, {}, &next_event};
     for (auto& e : ev) e = tm.get();
     AQ_CUDA(cudaMemsetAsync(w.film, 0, 16 * pixels * plan.replicas, st));
-    AQ_CUDA(cudaMemsetAsync(w.stats, 0, 8 * 16, st));
-    AQ_CUDA(cudaMemsetAsync(w.counters, 0, 4 * (kCntBucket0 + std::max<size_t>(nb, 1)), st));
+    AQ_CUDA(cudaMemsetAsync(w.counters, 0, w.counter_bytes, st));  // and the statistics behind them
     AQ_CUDA(cudaEventRecord(ev[0], st));
     uint64_t launches = 0;
     W.q_in = w.q[0];
@@ -1302,7 +1297,6 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     }
     AQ_CUDA(cudaEventRecord(ev[2], st));
     // Online training on this frame's records.
-    double loss = 0.0;
     int steps = 0;
     if (nrec > 0 && !visualize) {
         uint64_t a = 2654435761ull % nrec, b = 0x9E37ull % nrec;
@@ -1323,7 +1317,6 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
             nrc_train_step_dev(ctx, net, nw.t_x + 64 * r0, nw.t_target + 3 * r0, rows);
             launches += net.forward_tc ? 2 : 6;
         }
-        AQ_CUDA(cudaMemcpyAsync(&loss, net.loss, 8, cudaMemcpyDeviceToHost, st));
         // Aim the next frame's training-path fraction at the record budget.
         double per_path = ntp > 0 ? (double)pc[10] / (double)std::min<uint32_t>(ntp, P.max_train_paths) : 3.0;
         double want = (double)cfg.nrc_train_samples / std::max(per_path, 1.0);
@@ -1343,11 +1336,13 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     }
     if (!(flags & AQUA_RENDER_DEVICE_FILM))
         AQ_CUDA(cudaMemcpyAsync(rgb_out, w.out_rgb, 12 * pixels, cudaMemcpyDeviceToHost, st));
-    unsigned long long hs[16];
+    unsigned long long* const hs = ctx->pinned_stats;
     AQ_CUDA(cudaMemcpyAsync(hs, w.stats, 8 * 16, cudaMemcpyDeviceToHost, st));
+    nrc_read_back(ctx, net);
     AQ_CUDA(cudaStreamSynchronize(st));
     check_drained(hs[kStatPaths], pixels, cfg.spp);
     nrc_check_tc(ctx, net);
+    const double loss = *ctx->pinned_loss;  // of the last step
     if (stats) {
         memset(stats, 0, sizeof(*stats));
         float ms = 0.0f, q_ms = 0.0f, t_ms = 0.0f;
@@ -1518,8 +1513,9 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
         AQ_CUDA(cudaGetLastError());
         ++launches;
     }
-    unsigned long long hs[kNoAllocStats];
-    AQ_CUDA(cudaMemcpyAsync(hs, W.stats, sizeof(hs), cudaMemcpyDeviceToHost, st));
+    static_assert(kNoAllocStats == 16, "the context's page-locked statistics");
+    unsigned long long* const hs = ctx->pinned_stats;
+    AQ_CUDA(cudaMemcpyAsync(hs, W.stats, 8 * kNoAllocStats, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
     check_drained(hs[kStatPaths], pixels, cfg.spp);
     if (stats) {

@@ -137,14 +137,12 @@ void trace_rays(aqua_ctx* ctx, aqua_scene* sc, const aqua_ray* rays, size_t n, a
         {k_trace_user<true, kNodesFull>, k_trace_user<true, kNodesQuantized>, k_trace_user<true, kNodesWalk>}};
     const Walk walk = walks[any][walk_format(sc->ds)];
     const auto counted = any ? k_trace_count<true> : k_trace_count<false>;
-    int per_sm = 1;
-    if (count) AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, counted, 128, 0));
-    else AQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk, 128, 0));
+    const int per_sm = count ? resident_blocks(ctx, counted, 128) : resident_blocks(ctx, walk, 128);
     // A short queue is dealt to all warps (traverse_queue): down to one ray each.
     const size_t need = count ? (n + 127) / 128 : (n + 3) / 4;
-    int grid = (int)std::min<size_t>(need, (size_t)ctx->num_sms * (size_t)std::max(per_sm, 1));
-    EventPair ev;
-    AQ_CUDA(cudaEventRecord(ev.e[0], st));
+    int grid = (int)std::min<size_t>(need, (size_t)ctx->num_sms * (size_t)per_sm);
+    EventPair* ev = counts ? &timer(ctx) : nullptr;
+    if (ev) AQ_CUDA(cudaEventRecord(ev->e[0], st));
     if (count) {
         counted<<<grid, 128, 0, st>>>(sc->ds, d_rays, n, d_hits, d_stats);
         AQ_CUDA(cudaGetLastError());
@@ -156,16 +154,15 @@ void trace_rays(aqua_ctx* ctx, aqua_scene* sc, const aqua_ray* rays, size_t n, a
                                    reinterpret_cast<uint32_t*>(d_stats + 2));
         AQ_CUDA(cudaGetLastError());
     }
-    AQ_CUDA(cudaEventRecord(ev.e[1], st));
+    if (ev) AQ_CUDA(cudaEventRecord(ev->e[1], st));
     if (!dev) AQ_CUDA(cudaMemcpyAsync(out, d_hits, 16 * n, cudaMemcpyDeviceToHost, st));
-    unsigned long long hs[2] = {0, 0};
-    if (counts) AQ_CUDA(cudaMemcpyAsync(hs, d_stats, 16, cudaMemcpyDeviceToHost, st));
+    const bool read = counts && count;
+    if (read) AQ_CUDA(cudaMemcpyAsync(ctx->pinned_stats, d_stats, 16, cudaMemcpyDeviceToHost, st));
     AQ_CUDA(cudaStreamSynchronize(st));
-    const float ms = ev.ms();
     if (counts) {
-        counts->node_visits = hs[0];
-        counts->tri_tests = hs[1];
-        counts->kernel_ms = ms;
+        counts->node_visits = read ? ctx->pinned_stats[0] : 0;
+        counts->tri_tests = read ? ctx->pinned_stats[1] : 0;
+        counts->kernel_ms = ev->ms();
     }
 }
 
