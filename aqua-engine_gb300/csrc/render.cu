@@ -232,13 +232,11 @@ __global__ void k_raygen(DevScene S, WaveParams P, WavePtrs W) {
 
 // Raw cache features of a shading point (position, outgoing direction,
 // normal, roughness, diffuse albedo, specular F0).
-__device__ __forceinline__ void nrc_raw(float* o, v3 p, v3 wo, v3 n, float rough, v3 kd, v3 ks) {
-    o[0] = p.x; o[1] = p.y; o[2] = p.z;
-    o[3] = wo.x; o[4] = wo.y; o[5] = wo.z;
-    o[6] = n.x; o[7] = n.y; o[8] = n.z;
-    o[9] = rough;
-    o[10] = kd.x; o[11] = kd.y; o[12] = kd.z;
-    o[13] = ks.x; o[14] = ks.y; o[15] = ks.z;
+__device__ __forceinline__ void nrc_raw(float4* o, v3 p, v3 wo, v3 n, float rough, v3 kd, v3 ks) {
+    o[0] = make_float4(p.x, p.y, p.z, wo.x);
+    o[1] = make_float4(wo.y, wo.z, n.x, n.y);
+    o[2] = make_float4(n.z, rough, kd.x, kd.y);
+    o[3] = make_float4(kd.z, ks.x, ks.y, ks.z);
 }
 
 __device__ __forceinline__ void ltrain_add(float4* L, uint32_t id, v3 c) {
@@ -472,23 +470,18 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
                     if (!tag && query) {
                         uint32_t k = warp_append(&W.counters[kCntQuery], true);
                         W.q_pix[k] = make_float4(__int_as_float((int)pixel), thr.x, thr.y, thr.z);
-                        nrc_raw(W.q_raw + 16 * (size_t)k, p, wo, ns, m.b.y, kd, B.F0);
+                        nrc_raw(reinterpret_cast<float4*>(W.q_raw) + 4 * (size_t)k, p, wo, ns, m.b.y, kd, B.F0);
                         queried = true;
                     } else if (tag) {
                         float4 lb = W.ltrain[train_id];
                         W.lsnap[(size_t)train_id * (size_t)P.train_depth + depth] = lb;
                         uint32_t k = (int)depth < P.record_depth ? atomicAdd(&W.counters[kCntRecord], 1u) : 0xffffffffu;
                         if (k < P.max_records) {
-                            float r[24];
-                            nrc_raw(r, p, wo, ns, m.b.y, kd, B.F0);
-                            r[16] = thr.x; r[17] = thr.y; r[18] = thr.z;
-                            r[19] = lb.x; r[20] = lb.y; r[21] = lb.z;
-                            r[22] = __int_as_float((int)train_id);
-                            r[23] = __int_as_float((int)depth);
                             float4* dst = W.rec + 6 * (size_t)k;
-#pragma unroll
-                            for (int q = 0; q < 6; ++q)
-                                dst[q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                            nrc_raw(dst, p, wo, ns, m.b.y, kd, B.F0);
+                            dst[4] = make_float4(thr.x, thr.y, thr.z, lb.x);
+                            dst[5] = make_float4(lb.y, lb.z, __int_as_float((int)train_id),
+                                                 __int_as_float((int)depth));
                         }
                     }
                 }
@@ -1227,7 +1220,8 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     // the 1080p interior). Deep plain renders stay on three launches, where
     // the fused launch measured 2.3% slower (Cornell GGX 1024^2).
     const bool fused = !sorted;
-    const FusedKernel fused_k = fused_kernel(walk_format(S)), first_k = fused_kernel(first_format(S));
+    const FusedKernel fused_k = fused_kernel(walk_format(S));
+    const TraceKernel first_k = trace_kernel(first_format(S), false, false);
     int g_fused = fused ? grid_for(ctx, fused_k, 128, tune.blocks_per_sm) : 0;
 
     cudaEvent_t ev[4];
@@ -1259,7 +1253,12 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
             W.q_out = w.q[out];
             if (fused) {
                 const uint32_t sh_now = in ? kCntShadow1 : kCntShadow, sh_prev = in ? kCntShadow : kCntShadow1;
-                launch_chained(iter == 0 ? first_k : fused_k, g_fused, 128, 0, st, S, P, W, in, out, sh_prev, sh_now);
+                // No shadow rays yet in the first iteration: the plain kernel
+                // walks its camera rays faster than the fused one (a 1080p
+                // frame 2.99 -> 2.92 ms; the second iteration, too, in two
+                // launches: 2.96).
+                if (iter == 0) launch_chained(first_k, g_trace, 128, 0, st, S, P, W, in, out);
+                else launch_chained(fused_k, g_fused, 128, 0, st, S, P, W, in, out, sh_prev, sh_now);
                 launch_chained(shade_k, g_shade, 128, 0, st, S, P, W, in, out, sh_now);
                 launches += 2;
                 continue;
