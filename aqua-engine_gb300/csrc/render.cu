@@ -315,16 +315,67 @@ __global__ void __launch_bounds__(128, kTraceBlocks) k_trace_ext(DevScene S, Wav
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&W.stats[kStatExt], (unsigned long long)n);
 }
 
+// The hit and the path state of a thread's next queue entry, fetched into
+// shared memory while it shades the current one (cp.async; the slot of the
+// entry after that comes along). A thread reads only what it sent for, so no
+// barrier is involved. Without it k_shade waits for these loads in every
+// iteration: Cornell GGX 1024^2 at 256 spp 149.4 -> 146.3 ms, the Cornell box
+// 256^2 at 64 spp 2.21 -> 2.12 ms, loaded scene files 2.53 -> 2.49, a cached
+// 1080p frame 2.935 -> 2.91, the 1080p interior the same. Not taken: throughput
+// and direction as well (Cornell 146.5, the interior 1% slower: its L1
+// shrinks), two buffers (16 KB a block move the shared-memory carve-out between
+// kernels: 161 ms), the first entry loaded directly (149.2).
+struct ShadeAhead {
+    uint32_t idx[2][128];
+    uint4 state[2][128];
+    static __device__ __forceinline__ uint32_t addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+    __device__ __forceinline__ void fetch(const WavePtrs& W, uint32_t s) {
+        const uint32_t t = threadIdx.x;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(addr(&state[0][t])), "l"(W.hit + s)
+                     : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(addr(&state[1][t])), "l"(W.pst + s)
+                     : "memory");
+    }
+    __device__ __forceinline__ void fetch_slot(uint32_t k, const uint32_t* q) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(addr(&idx[k & 1u][threadIdx.x])), "l"(q)
+                     : "memory");
+    }
+    // Entry i of n is the thread's first.
+    __device__ __forceinline__ void start(const WavePtrs& W, uint32_t i, uint32_t n, uint32_t stride) {
+        if (i >= n) return;
+        const uint32_t s = W.q_in[i];
+        idx[0][threadIdx.x] = s;
+        fetch(W, s);
+        if (i + stride < n) fetch_slot(1, W.q_in + i + stride);
+    }
+    // Entry i of n, the thread's k-th: its slot, hit and path state.
+    __device__ __forceinline__ uint32_t take(const WavePtrs& W, uint32_t k, uint32_t i, uint32_t n, uint32_t stride,
+                                             float4& hit, uint4& pst) {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        const uint32_t s = idx[k & 1u][threadIdx.x];
+        const uint4 h = state[0][threadIdx.x];
+        hit = make_float4(__uint_as_float(h.x), __uint_as_float(h.y), __uint_as_float(h.z), __uint_as_float(h.w));
+        pst = state[1][threadIdx.x];
+        if (i + stride < n) fetch(W, idx[(k + 1u) & 1u][threadIdx.x]);
+        if (i + 2u * stride < n) fetch_slot(k, W.q_in + i + 2u * stride);
+        return s;
+    }
+};
+
 // NRC: paths that are not training paths stop at bounce P.query_depth and
 // queue a cache query (pixel, throughput, raw features); training paths run
 // on and record every bounce (raw features, throughput, radiance gathered
 // so far) so that the radiance leaving each of their vertices becomes a
 // training target once the path is complete.
-template <bool SORTED, bool NRC = false, bool FULL = false>
+// AHEAD (unsorted queues that outgrow the grid, shade_kernel): the next entry's
+// loads run ahead (ShadeAhead). With one entry per thread there is nothing to send for,
+// and going through shared memory costs a 64 x 64 thumbnail 1% (207.5 -> 210 us).
+template <bool SORTED, bool NRC, bool FULL, bool AHEAD>
 __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, WavePtrs W, uint32_t cnt_in,
                                                uint32_t cnt_out, uint32_t cnt_sh) {
     __shared__ float lut[256];
-    __shared__ uint32_t prefix[257];
+    __shared__ uint32_t prefix[SORTED ? 257 : 1];
+    __shared__ ShadeAhead ahead;
     if (S.n_texs > 0) fill_srgb_lut(lut);
     grid_dep_wait();
     grid_dep_launch();
@@ -348,16 +399,19 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
     uint32_t* out_cnt = &W.counters[cnt_out];
     unsigned long long done_paths = 0;
     __shared__ uint32_t s_warp[2][5];
+    const uint32_t stride = gridDim.x * blockDim.x;
     uint32_t turn = 0;
+    if (AHEAD) ahead.start(W, blockIdx.x * blockDim.x + threadIdx.x, n, stride);
     // The whole block iterates together (the out-queue append is per block).
-    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+    for (uint32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
         const uint32_t i = i0 + threadIdx.x;
         uint32_t s = 0;
         bool cont = false;
         if (i < n) {
         // With sorted queues the bucket is the material, so its parameters
         // load alongside the path state instead of after the triangle.
-        float4 mat_a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), mat_b = mat_a;
+        float4 mat_a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), mat_b = mat_a, h;
+        uint4 ps;
         if (SORTED) {
             uint32_t lo = 0, hi = P.nb - 1;
             while (lo < hi) {  // last bucket b with prefix[b] <= i
@@ -371,12 +425,16 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
                 mat_a = ldg_(mp);
                 mat_b = ldg_(mp + 1);
             }
+        } else if (AHEAD) {
+            s = ahead.take(W, turn, i, n, stride, h, ps);
         } else {
             s = W.q_in[i];
         }
-        uint4 ps = W.pst[s];
+        if (!AHEAD) {
+            ps = W.pst[s];
+            h = W.hit[s];
+        }
         float4 tpv = W.tp[s];
-        float4 h = W.hit[s];
         uint32_t j = ps.z, depth = ps.w & 0xffu, tag = ps.w & ~0xffu;
         const uint32_t train_id = (tag >> 8) - 1u;  // valid when tag != 0
         const PathId pid = path_id(P, s, j);
@@ -549,8 +607,8 @@ __global__ void __launch_bounds__(128, 6) k_shade(DevScene S, WaveParams P, Wave
             }
         }
         }
-        const uint32_t k = block_append(out_cnt, cont, s_warp[turn]);
-        turn ^= 1u;
+        const uint32_t k = block_append(out_cnt, cont, s_warp[turn & 1u]);
+        ++turn;
         if (cont) W.q_out[k] = s;
     }
     for (int o = 16; o > 0; o >>= 1) done_paths += __shfl_down_sync(0xffffffffu, done_paths, o);
@@ -735,6 +793,7 @@ void workspace_release(aqua_ctx* ctx) {
 // The traversal kernels of a scene's node format (the counting ones walk the
 // canonical tree, whatever the format).
 using TraceKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t);
+using ShadeKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t, uint32_t);
 using ShadowKernel = void (*)(DevScene, WaveParams, WavePtrs);
 using FusedKernel = void (*)(DevScene, WaveParams, WavePtrs, uint32_t, uint32_t, uint32_t, uint32_t);
 
@@ -772,6 +831,17 @@ template <class K>
 static int grid_for(aqua_ctx* ctx, K kernel, int block, int blocks_per_sm) {
     const int per_sm = blocks_per_sm > 0 ? blocks_per_sm : resident_blocks(ctx, kernel, block);
     return ctx->num_sms * per_sm;
+}
+
+// Loading ahead (ShadeAhead) pays from the second queue entry of a thread on:
+// for renders whose slots outnumber the grid's threads (both sides measured at
+// k_shade).
+template <bool NRC>
+static ShadeKernel shade_kernel(aqua_ctx* ctx, bool sorted, bool full, size_t slots, int block, int blocks_per_sm) {
+    if (sorted) return full ? k_shade<true, NRC, true, false> : k_shade<true, NRC, false, false>;
+    const ShadeKernel plain = full ? k_shade<false, NRC, true, false> : k_shade<false, NRC, false, false>;
+    if (slots <= (size_t)grid_for(ctx, plain, block, blocks_per_sm) * (size_t)block) return plain;
+    return full ? k_shade<false, NRC, true, true> : k_shade<false, NRC, false, true>;
 }
 
 namespace {
@@ -922,8 +992,7 @@ void render_path(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, 
     const TraceKernel trace_k = trace_kernel(walk_format(S), sorted, count);
     const TraceKernel first_k = trace_kernel(first_format(S), sorted, count);
     const bool full = S.mext != nullptr;  // some material sets the full model's lobes
-    auto shade_k = full ? (sorted ? k_shade<true, false, true> : k_shade<false, false, true>)
-                        : (sorted ? k_shade<true> : k_shade<false>);
+    const ShadeKernel shade_k = shade_kernel<false>(ctx, sorted, full, slots, bs, tune.blocks_per_sm);
     const ShadowKernel shadow_k = shadow_kernel(S, count, false);
     int g_trace = grid_for(ctx, trace_k, bt, tune.blocks_per_sm);
     int g_shade = grid_for(ctx, shade_k, bs, tune.blocks_per_sm);
@@ -1206,8 +1275,12 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
     W.spread = nw.spread;
 
     const TraceKernel trace_k = trace_kernel(walk_format(S), sorted, false);
-    auto shade_k = S.mext ? (sorted ? k_shade<true, true, true> : k_shade<false, true, true>)
-                          : (sorted ? k_shade<true, true> : k_shade<false, true>);
+    // The queues are full up to vertex 2, where most paths query; past it they
+    // are short, and loading ahead costs more than it gives (a 480 x 270 frame
+    // 1.34 -> 1.36 ms).
+    const ShadeKernel shade_full =
+        shade_kernel<true>(ctx, sorted, S.mext != nullptr, slots, 128, tune.blocks_per_sm);
+    const ShadeKernel shade_k = shade_kernel<true>(ctx, sorted, S.mext != nullptr, 0, 128, tune.blocks_per_sm);
     const ShadowKernel shadow_k = shadow_kernel(S, false, true);
     int g_trace = grid_for(ctx, trace_k, 128, tune.blocks_per_sm);
     int g_shade = grid_for(ctx, shade_k, 128, tune.blocks_per_sm);
@@ -1259,7 +1332,7 @@ void render_nrc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cfg, c
                 // launches: 2.96).
                 if (iter == 0) launch_chained(first_k, g_trace, 128, 0, st, S, P, W, in, out);
                 else launch_chained(fused_k, g_fused, 128, 0, st, S, P, W, in, out, sh_prev, sh_now);
-                launch_chained(shade_k, g_shade, 128, 0, st, S, P, W, in, out, sh_now);
+                launch_chained(iter < 2 ? shade_full : shade_k, g_shade, 128, 0, st, S, P, W, in, out, sh_now);
                 launches += 2;
                 continue;
             }
@@ -1472,7 +1545,7 @@ void render_noalloc(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg& cf
     AQ_CUDA(cudaMemsetAsync(W.stats, 0, 8 * kNoAllocStats, st));
 
     const TraceKernel trace_k = trace_kernel(walk_format(S), false, false);
-    auto shade_k = S.mext ? k_shade<false, false, true> : k_shade<false>;
+    const ShadeKernel shade_k = shade_kernel<false>(ctx, false, S.mext != nullptr, slots, 128, 0);
     const ShadowKernel shadow_k = shadow_kernel(S, false, false);
     int g_trace = grid_for(ctx, trace_k, 128, 0);
     int g_shade = grid_for(ctx, shade_k, 128, 0);
