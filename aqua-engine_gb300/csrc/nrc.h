@@ -40,8 +40,10 @@ constexpr int kNrcRaw = 16;  // raw vertex features, floats
 // Tensor-core weight images, bf16 in the no-swizzle K-major operand layout
 // (element (r, k) of an R-row tile at (k / 8) R 16 + r 16 + (k % 8) 2 bytes).
 // Forward image: W1..W5 as 64-row tiles (rows = outputs, K = inputs), then
-// W6 padded to 16 rows. Backward image: W6^T (64 rows = inputs, K = 16
-// outputs, 3 used), then W5^T..W2^T. Padding stays zero.
+// W6 padded to 16 rows; padding stays zero. The training kernel reads the
+// transposes from it through the MMA's transposed operand form. Backward image
+// (a layout the device no longer stores): W6^T (64 rows = inputs, K = 16
+// outputs, 3 used), then W5^T..W2^T.
 constexpr int kNrcTcLayerBytes = 64 * 64 * 2;  // 8 KB
 constexpr int kNrcTcOutRows = 16;
 constexpr int kNrcTcBwdW6Bytes = 64 * 16 * 2;  // 2 KB

@@ -364,8 +364,8 @@ SHADE_TRAFFIC = {
 
 def trace_roofline(ctx, scene, cfg, film_ptr, hbm_peak, peak_src, l2_gbs, count_spp, traffic=None):
     """Roofline of k_trace_ext on one scene: algorithmic bytes per ray from a
-    counting pass at count_spp (node visits x NODE_BYTES + triangle tests x
-    48 + 48 B of ray and hit), times the rays per launch of a full render,
+    counting pass at count_spp (node visits x the bytes of a node as the
+    scene is walked + triangle tests x 48 + 48 B of ray and hit), times the rays per launch of a full render,
     over the mean launch time from CUDA events around every 8th launch of
     that render (RENDER_STAGE_TIMING; an extra render outside the timed
     steps)."""
@@ -373,14 +373,15 @@ def trace_roofline(ctx, scene, cfg, film_ptr, hbm_peak, peak_src, l2_gbs, count_
 
     ccfg = ctx.integrator(spp=count_spp, max_depth=cfg.max_depth, rr_depth=cfg.rr_depth, seed=cfg.seed)
     cst = ctx.render_device(scene, ccfg, film_ptr, flags=aqua.RENDER_COUNT)
-    bytes_per_ray = (cst.node_visits * NODE_BYTES + cst.tri_tests * 48) / max(cst.ext_rays, 1) + 48
+    node_bytes = WALK_NODE_BYTES if scene.info().num_bvh_nodes >= WALK_NODES_FROM else NODE_BYTES
+    bytes_per_ray = (cst.node_visits * node_bytes + cst.tri_tests * 48) / max(cst.ext_rays, 1) + 48
     st = ctx.render_device(scene, cfg, film_ptr, flags=aqua.RENDER_STAGE_TIMING)
     rays_per_launch = st.ext_rays / max(st.iterations, 1)
     avg_launch_s = st.trace_ms * 1e-3 / max(st.trace_launches, 1)
     achieved = bytes_per_ray * rays_per_launch / avg_launch_s / 1e9
     out = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
            "peak_source": peak_src, "kernel": "k_trace_ext (closest-hit BVH traversal)",
-           "bytes_per_ray": bytes_per_ray, "rays_per_launch": rays_per_launch,
+           "bytes_per_ray": bytes_per_ray, "node_bytes": node_bytes, "rays_per_launch": rays_per_launch,
            "avg_launch_us": avg_launch_s * 1e6, "frac_of_l2_copy": achieved / l2_gbs if l2_gbs else None,
            "node_visits_per_ray": cst.node_visits / max(cst.ext_rays, 1),
            "tri_tests_per_ray": cst.tri_tests / max(cst.ext_rays, 1), "counting_spp": count_spp,
@@ -430,6 +431,7 @@ NRC_INFER_WORKLOAD = {"workload": "nrc-inference-16777216-rows", "rows": 1 << 24
                       "inputs": "encoded from uniform random vertex features (positions in the unit box, "
                                 "unit directions and normals, albedos), seed 21"}
 NODE_BYTES = 112  # a four-wide node visit reads seven 16-byte words (its counts word is not read)
+WALK_NODE_BYTES, WALK_NODES_FROM = 64, 150_000  # larger trees are walked through 64-byte nodes (csrc/internal.h)
 NRC_FLOP_PER_ROW = 2 * (5 * 64 * 64 + 3 * 64)  # 41,344 useful multiply-adds x 2
 NRC_BYTES_PER_ROW = 128 + 12                   # bf16 input row + fp32 output
 
@@ -509,12 +511,12 @@ def run_nrc_training_metric(ctx, peak: float, peak_src: str, warmup: int = 5, st
         del raw, x, tgt
     big = out[str(batches[-1])]
     return {"config": {"workload": "nrc-train-step", "batches": list(batches),
-                       "step": "forward (tcgen05) + backward (tcgen05) + weight gradients (tcgen05) + Adam",
+                       "step": "one tcgen05 launch (forward, backward, weight gradients) + Adam",
                        "flop_per_row": NRC_TRAIN_FLOP_PER_ROW},
             "unit": "Mrows/s", "value": big["rows_per_s"] / 1e6, "steps": steps, "warmup": warmup, "by_batch": out,
             "roofline": {"bound": "tensor", "achieved": big["tflops"], "peak": peak, "unit": "TFLOP/s",
                          "frac": big["frac"], "peak_source": peak_src,
-                         "kernel": f"one training step at {batches[-1]} rows (4 launches + weight packing)"}}
+                         "kernel": f"one training step at {batches[-1]} rows (2 launches)"}}
 
 
 BATCH_WORKLOAD = {"workload": "batch-64-jobs-4-scenes",

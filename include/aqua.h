@@ -196,7 +196,7 @@ typedef struct aqua_scene_info {
     int32_t num_triangles, num_materials, num_lights, num_textures;
     int32_t num_meshes, num_bvh_nodes; /* nodes of the four-wide BVH     */
     int32_t bvh_depth, max_leaf_size;  /* wide nodes on the longest path  */
-    uint64_t device_bytes;   /* device memory held by the scene             */
+    uint64_t device_bytes;   /* device memory held by the scene, its walk nodes included */
     uint64_t upload_bytes;   /* bytes copied host->device by one upload     */
     float env[3];            /* constant radiance seen by escaping rays     */
     int32_t bvh_format;      /* AQUA_BVH_FULL or AQUA_BVH_QUANTIZED: the node
@@ -401,9 +401,10 @@ AQUA_API aqua_status aqua_autotune(aqua_ctx* ctx, aqua_scene* scene,
 /* Renders n jobs (views of up to n scenes, uneven resolutions and spp; at
  * most 1024 jobs) in one persistent launch replayed from a captured CUDA
  * graph (tuning->use_graph, on when tuning is NULL). Each lane owns one
- * pixel and runs its samples one path after another; idle lanes take the
- * next pixels from a global queue on which the jobs are laid out shortest
- * first (pixels x spp), so small jobs complete early. Every job's image
+ * pixel's samples, or a run of them in batches with few pixels, and traces
+ * them one path after another; idle lanes take the next ones from a global
+ * queue on which the jobs are laid out shortest first (pixels x spp), so small
+ * jobs complete early. Every job's image
  * equals aqua_render's. rgb_out of each job is a device buffer. stats->job_ms,
  * when non-NULL, receives each job's completion time from the start of the
  * launch (device clock). tuning->block_trace = threads per block (64, 128,
