@@ -208,6 +208,20 @@ __device__ __forceinline__ void add_product(float4* sum, v3 a, v3 b) {
     *sum = make_float4(r.x, r.y, r.z, f.w);
 }
 
+// Requests a line into L2. The shadow records and films of 16M paths stream
+// from DRAM, and a lane that waits for its ray, or for the film behind it, holds
+// up its warp: k_shadow asks for the records kRaysAhead further down the queue
+// when it loads one, and for its own contribution and film entry when the walk
+// begins. Cornell GGX 1024^2 at 256 spp 146.05 -> 145.0 ms, the Cornell box 256^2
+// at 64 spp 2.123 -> 2.107, loaded scene files 2.489 -> 2.479, the interior at
+// 1080p 39.76 -> 39.58. (The same for extension rays: another 0.5 ms on Cornell, but cached
+// frames 0.3% slower. Adding to the film with vector reductions, which wait for
+// nothing: 178.8 ms.) Queues up to kStreamFrom records are still in L2.
+constexpr uint32_t kRaysAhead = 65536, kStreamFrom = 2621440;
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+
 __device__ __forceinline__ void film_add(float4* film, uint32_t pixel, v3 c) {
     float4 f = film[pixel];
     f.x += c.x; f.y += c.y; f.z += c.z;
@@ -641,10 +655,17 @@ __global__ void __launch_bounds__(128, kTraceBlocks) k_shadow(DevScene S, WavePa
     uint32_t nodes = 0, tris = 0;
     auto finish = [&](uint32_t i, const TraceResult& r) { shadow_done<NRC>(P, W, i, r); };
     if (!COUNT) {
+        const uint32_t ahead_end = n > kStreamFrom ? n - kRaysAhead : 0u;
         traverse_queue<kQueueAny, NODES>(
             S, n, &W.counters[kCntFetchShadow],
             [&](uint32_t i, v3& o, v3& d, float& tmin, float& tmax) -> uint32_t {
                 float4 ro = W.sh_o[i], rd = W.sh_d[i];
+                if (i < ahead_end) {
+                    prefetch_l2(W.sh_o + i + kRaysAhead);
+                    prefetch_l2(W.sh_d + i + kRaysAhead);
+                }
+                prefetch_l2(W.sh_c + i);
+                prefetch_l2(W.film + (uint32_t)__float_as_int(ro.w));
                 o = f3(ro);
                 d = f3(rd);
                 tmin = 0.0f;
