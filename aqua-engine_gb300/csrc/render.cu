@@ -214,9 +214,10 @@ __device__ __forceinline__ void add_product(float4* sum, v3 a, v3 b) {
 // when it loads one, and for its own contribution and film entry when the walk
 // begins. Cornell GGX 1024^2 at 256 spp 146.05 -> 145.0 ms, the Cornell box 256^2
 // at 64 spp 2.123 -> 2.107, loaded scene files 2.489 -> 2.479, the interior at
-// 1080p 39.76 -> 39.58. (The same for extension rays: another 0.5 ms on Cornell, but cached
-// frames 0.3% slower. Adding to the film with vector reductions, which wait for
-// nothing: 178.8 ms.) Queues up to kStreamFrom records are still in L2.
+// 1080p 39.76 -> 39.58. (The same for extension rays: another 0.5 ms on Cornell,
+// but cached frames 0.3% slower. Adding to the film with vector reductions,
+// which wait for nothing: 178.8 ms.) Queues up to kStreamFrom records are still
+// in L2.
 constexpr uint32_t kRaysAhead = 65536, kStreamFrom = 2621440;
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
