@@ -205,7 +205,14 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     for (int i = 0; i < 3; ++i) ds.env[i] = h.env[i];
     ds.cam = dev_camera(h.cam);
     scene_upload(ctx, s);
-    if (use_walk) build_walk_nodes(ctx, ds, (float4*)(d + total));
+    if (use_walk) {
+        // The load ends with the nodes in place: any context may walk them next,
+        // on a stream that does not wait for this one.
+        s->uploaded = false;
+        build_walk_nodes(ctx, ds, (float4*)(d + total));
+        AQ_CUDA(cudaStreamSynchronize(ctx->stream));
+        s->uploaded = true;
+    }
 }
 
 void scene_upload(aqua_ctx* ctx, aqua_scene* s) {
