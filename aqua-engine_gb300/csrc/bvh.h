@@ -64,6 +64,11 @@ struct FlatBvh {
     int num_nodes() const { return (int)(nodes.size() / kBvhNodeFloats); }
 };
 
+// Whether a walk through the tree's walk nodes (walk_nodes.h) fits the stack
+// whatever the ray: their empty slots can be accepted, so a node may push three
+// entries even where it has only two children, which max_stack counts as one.
+inline bool walk_stack_fits(const FlatBvh& bvh) { return (kBvhWidth - 1) * bvh.depth <= kBvhStackSize; }
+
 // verts: 9 floats per triangle.
 FlatBvh build_bvh(const float* verts, size_t num_tris);
 

@@ -105,7 +105,7 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
         if (m.specular_tint > 0.0f || m.sheen > 0.0f || m.clearcoat > 0.0f || m.transmission > 0.0f) full_bsdf = true;
     size_t total = align256(o_mext + (full_bsdf ? 32 * h.mats.size() : 0));
     // Walk nodes follow the uploaded image; the device derives them.
-    bool use_walk = !use_q && nn >= kWalkNodesFrom && !ctx->host_only;
+    bool use_walk = !use_q && nn >= kWalkNodesFrom && walk_stack_fits(s->bvh) && !ctx->host_only;
     for (int a = 0; a < 3; ++a)  // a walk node's frame must stay within the float range
         use_walk = use_walk && std::fabs(s->bvh.lo[a]) < 1e15f && std::fabs(s->bvh.hi[a]) < 1e15f;
     free_staging(s);

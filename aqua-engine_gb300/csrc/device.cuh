@@ -8,6 +8,7 @@
 
 #include "aq_math.h"
 #include "bvh.h"
+#include "walk_nodes.h"
 
 namespace aq {
 
@@ -33,7 +34,7 @@ struct DevCamera {
 };
 struct DevScene {
     const float4* __restrict__ nodes;  // 8 words per four-wide node, or 4 per quantized node (bvh.h)
-    const float4* __restrict__ wnodes; // 4 words per walk node (visit_walk); null for small trees and with qbvh
+    const float4* __restrict__ wnodes; // 4 words per walk node (load_walk); null for small trees and with qbvh
     const float4* __restrict__ tris;   // 3 words per triangle, leaf order
     const float2* __restrict__ uvs;    // 3 per triangle, leaf order
     const DevMaterial* __restrict__ mats;
@@ -168,56 +169,16 @@ __device__ __forceinline__ Children load_quantized(const DevScene& S, int32_t no
     return c;
 }
 
-// Walk node (k_walk_nodes, 64 bytes): the child boxes rounded outward to
-// 8-bit offsets in the node's frame, like a quantized node, but tested
-// without decoding the planes. Word 0 = (origin.xyz, Sx), word 1 = links,
-// words 2-3 = (lo.x, hi.x, lo.y, hi.y), (lo.z, hi.z, Sy, Sz), one byte per
-// child, S = 2^15 x the step s of the axis (a power of two). One byte
-// permute makes the float 1 + q 2^-15, and with b = (origin - o) / d and
-// A = S / d one multiply-add gives the distance to the plane:
-//   (1 + q 2^-15) A + (b - A) = b + q s / d.
-// The rounding errors of a plane's distance stay below
-// 5 x 2^-24 (|b| + |A|); near planes are moved back and far planes forward
-// by 8 x 2^-24 (|b| + |A|) (1/64 of a step at most), which also covers the
-// rounding of slab_entry on the exact planes. So every box that slab_entry
-// accepts is accepted here, and a walk whose hits are
-// confirmed (walk_confirmed) finds what the full-precision walk finds.
-// The ray's signs choose the near and far words, six selections per node
-// instead of two min/max per plane pair and child: the arithmetic costs what
-// the full-precision node's does, from 64 bytes and two loads instead of 112
-// bytes and four. The walk of large trees is bound by its node fetches
-// (L1 data pipe 71% busy on the 1.15M-triangle interior): 2.07M rays against
-// it 540 -> 520 us, its 1080p render at 8 spp 49.1 -> 43.9 ms.
-__device__ __forceinline__ float walk_byte(uint32_t word, int k) {
-    return __uint_as_float(__byte_perm(word, 0x3F800000u, 0x7604u | ((uint32_t)k << 4)));
-}
+// Walk node (64 bytes, two 256-bit loads; walk_nodes.h).
 __device__ __forceinline__ Children load_walk(const DevScene& S, int32_t node, const RayPre& rp, float tfar) {
     const float4* np = S.wnodes + 4 * (size_t)node;
     float4 w0, w1, w2, w3;
     ldg2x4(np, w0, w1);
     ldg2x4(np + 2, w2, w3);
-    constexpr float kPad = 4.76837158203125e-7f;  // 2^-21
-    const float bx = mul_rn(sub_rn(w0.x, rp.o.x), rp.invd.x), by = mul_rn(sub_rn(w0.y, rp.o.y), rp.invd.y),
-                bz = mul_rn(sub_rn(w0.z, rp.o.z), rp.invd.z);
-    const float ax = mul_rn(w0.w, rp.invd.x), ay = mul_rn(w3.z, rp.invd.y), az = mul_rn(w3.w, rp.invd.z);
-    const float mx = add_rn(fabsf(bx), fabsf(ax)), my = add_rn(fabsf(by), fabsf(ay)), mz = add_rn(fabsf(bz), fabsf(az));
-    const float dx = sub_rn(bx, ax), dy = sub_rn(by, ay), dz = sub_rn(bz, az);
-    const float bnx = fmaf(-kPad, mx, dx), bfx = fmaf(kPad, mx, dx), bny = fmaf(-kPad, my, dy),
-                bfy = fmaf(kPad, my, dy), bnz = fmaf(-kPad, mz, dz), bfz = fmaf(kPad, mz, dz);
-    const uint32_t lx = __float_as_uint(w2.x), hx = __float_as_uint(w2.y), ly = __float_as_uint(w2.z),
-                   hy = __float_as_uint(w2.w), lz = __float_as_uint(w3.x), hz = __float_as_uint(w3.y);
-    const bool ix = rp.invd.x < 0.0f, iy = rp.invd.y < 0.0f, iz = rp.invd.z < 0.0f;
-    const uint32_t qnx = ix ? hx : lx, qfx = ix ? lx : hx, qny = iy ? hy : ly, qfy = iy ? ly : hy,
-                   qnz = iz ? hz : lz, qfz = iz ? lz : hz;
+    const WalkBoxes w{w0.x, w0.y, w0.z, w0.w, w3.z, w3.w, __float_as_uint(w2.x), __float_as_uint(w2.y),
+                      __float_as_uint(w2.z), __float_as_uint(w2.w), __float_as_uint(w3.x), __float_as_uint(w3.y)};
     float t[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float n = fmaxf(fmaxf(fmaf(walk_byte(qnx, k), ax, bnx), fmaf(walk_byte(qny, k), ay, bny)),
-                              fmaxf(fmaf(walk_byte(qnz, k), az, bnz), rp.tmin));
-        const float f = fminf(fminf(fmaf(walk_byte(qfx, k), ax, bfx), fmaf(walk_byte(qfy, k), ay, bfy)),
-                              fminf(fmaf(walk_byte(qfz, k), az, bfz), tfar));
-        t[k] = n <= mul_rn(f, kSlabFarScale) ? n : INFINITY;
-    }
+    walk_entries(w, rp, tfar, t);
     Children c;
     c.t0 = t[0], c.t1 = t[1], c.t2 = t[2], c.t3 = t[3];
     c.c0 = __float_as_int(w1.x), c.c1 = __float_as_int(w1.y), c.c2 = __float_as_int(w1.z), c.c3 = __float_as_int(w1.w);

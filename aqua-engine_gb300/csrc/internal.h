@@ -292,7 +292,7 @@ void dev_free(DevBuf& b);
 // where the tree's memory footprint matters.
 constexpr size_t kQuantizeAbove = (size_t)8 << 30;
 void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh = true);
-// Walk nodes (device.cuh, load_walk) of the scene's full-precision nodes:
+// Walk nodes (walk_nodes.h) of the scene's full-precision nodes:
 // 64 bytes per node, written on the context's stream.
 void build_walk_nodes(aqua_ctx* ctx, const DevScene& S, float4* out);
 // The node format a scene's rays walk (kNodes*).

@@ -54,43 +54,15 @@ __global__ void __launch_bounds__(128) k_trace_count(DevScene S, const float4* _
     }
 }
 
-// One thread per node: the walk node of full-precision node k. All steps
-// are exact: a plane lo + q 2^e of floats lo and 8-bit q needs at most 41
-// bits (2^e is at least an 256th of an ulp of the larger plane), so the
-// doubles below hold it.
+// One thread per node: the walk node of full-precision node k (walk_nodes.h).
 __global__ void k_walk_nodes(const float4* __restrict__ nodes, int32_t n, float4* __restrict__ out) {
     const int32_t k = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     if (k >= n) return;
     const float* w = reinterpret_cast<const float*>(nodes + 8 * (size_t)k);
     const int32_t* link = reinterpret_cast<const int32_t*>(w + 24);
     float org[3], step[3];
-    uint32_t lo_bytes[3] = {0, 0, 0}, hi_bytes[3] = {0, 0, 0};
-    for (int a = 0; a < 3; ++a) {
-        float lo = INFINITY, hi = -INFINITY;
-        for (int c = 0; c < 4; ++c)
-            if (link[c] != ~0) {
-                lo = fminf(lo, w[8 * a + c]);
-                hi = fmaxf(hi, w[8 * a + 4 + c]);
-            }
-        if (!(lo <= hi)) lo = hi = 0.0f;  // no children (not produced by the builder)
-        int e = -100;
-        if (hi > lo) {  // smallest step whose 255 multiples reach hi
-            e = max(-100, ilogb(((double)hi - (double)lo) / 255.0));
-            if (ldexp(255.0, e) < (double)hi - (double)lo) ++e;
-        }
-        const double s = ldexp(1.0, e);
-        org[a] = lo;
-        step[a] = (float)ldexp(1.0, e + 15);
-        for (int c = 0; c < 4; ++c) {
-            uint32_t ql = 255, qh = 0;  // empty slot: a box no ray enters
-            if (link[c] != ~0) {
-                ql = (uint32_t)floor(((double)w[8 * a + c] - (double)lo) / s);
-                qh = (uint32_t)ceil(((double)w[8 * a + 4 + c] - (double)lo) / s);
-            }
-            lo_bytes[a] |= ql << (8 * c);
-            hi_bytes[a] |= qh << (8 * c);
-        }
-    }
+    uint32_t lo_bytes[3], hi_bytes[3];
+    for (int a = 0; a < 3; ++a) walk_axis(w + 8 * a, w + 8 * a + 4, link, org[a], step[a], lo_bytes[a], hi_bytes[a]);
     float4* o = out + 4 * (size_t)k;
     o[0] = make_float4(org[0], org[1], org[2], step[0]);
     o[1] = nodes[8 * (size_t)k + 6];
