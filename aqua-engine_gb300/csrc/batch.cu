@@ -25,6 +25,7 @@
 #include <map>
 #include <vector>
 
+#include "batch_units.h"
 #include "internal.h"
 #include "shading.cuh"
 
@@ -412,42 +413,6 @@ struct BatchResult {
     uint64_t paths = 0, ext = 0, shadow = 0;
     std::vector<unsigned long long> clocks;
 };
-
-// Splits the pixels' samples into units (DevJob) for about `lanes` lanes (the
-// GPU's at the default launch shape, so that an image's rounding does not
-// depend on the shape). A pixel's samples run one after another on one lane, so the last
-// pixels of a small batch kept a few lanes busy long after the others had
-// run dry (a 51 x 145 view of the interior at 43 spp took 19 ms alone); units
-// short enough that each lane takes kUnitsPerLane of them bound that tail
-// (four views of up to 128^2 at 6 spp 2.41 -> 0.81 ms, ten of up to 300^2 at 16
-// spp 7.56 -> 3.31, twenty of up to 512^2 at 48 spp 41.4 -> 35.7). A large
-// batch keeps whole pixels.
-// Returns the items; pixels and partial sums of the split jobs by reference.
-constexpr uint64_t kBatchLanes = 768;  // per SM
-constexpr uint64_t kUnitsPerLane = 64;  // 16, 32 and 128: within 4%
-
-static uint32_t split_jobs(std::vector<DevJob>& jobs, uint64_t lanes, bool split, uint32_t& split_pixels,
-                           uint32_t& parts) {
-    uint64_t paths = 0;
-    for (const DevJob& j : jobs) paths += (uint64_t)j.pixels * (uint64_t)j.spp;
-    const uint64_t run = std::max<uint64_t>(1, paths / (lanes * kUnitsPerLane));
-    uint32_t items = 0;
-    split_pixels = parts = 0;
-    for (DevJob& j : jobs) {
-        j.unit_spp = split && run < (uint64_t)j.spp ? (uint32_t)run : (uint32_t)j.spp;
-        j.units = ((uint32_t)j.spp + j.unit_spp - 1) / j.unit_spp;
-        j.item_begin = items;
-        j.part_begin = j.done_begin = 0;
-        if (j.units > 1) {
-            j.part_begin = parts;
-            j.done_begin = split_pixels;
-            parts += j.units * j.pixels;
-            split_pixels += j.pixels;
-        }
-        items += j.units * j.pixels;
-    }
-    return items;
-}
 
 static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::vector<DevScene>& scenes,
                                const aqua_tuning& tune, bool split) {
