@@ -11,8 +11,9 @@
 // lane traces the path's extension and shadow rays one at a time and keeps
 // its walk between rounds, so lanes whose ray is done shade while others walk
 // on. Contributions are summed in the wavefront's order (emission, then
-// next-event estimation, bounce after bounce, sample after sample; a split
-// pixel's runs in order), so a job's image matches aqua_render's. The lane that
+// next-event estimation, bounce after bounce), and samples in an order that the
+// job alone sets (batch_units.h), so a job's image matches aqua_render's up to
+// the order of the sums and has the same bits in any company. The lane that
 // finishes a job's last pixel stamps the device clock, giving per-job
 // latencies.
 //
@@ -215,8 +216,8 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
     uint32_t n_ext = 0, n_sh = 0, n_paths = 0;
     bool have = false, walking = false, drained = false;
     int job = 0;
-    uint32_t pixel = 0, sample = 0, sample_end = 0;
-    v3 sum = mk(0.0f, 0.0f, 0.0f);
+    uint32_t pixel = 0, sample = 0, run_end = 0;
+    v3 sum = mk(0.0f, 0.0f, 0.0f), total = mk(0.0f, 0.0f, 0.0f);  // of the run; of an unsplit pixel's runs before
     LanePath P;
     P.shadow = false;
     // The ray in flight.
@@ -245,32 +246,41 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                     alive = shade_hit<FULL>(scenes[J.scene], J.max_depth, J.rr_depth, lut, r, P, sum);
                     alive = alive || P.shadow;
                 }
-                if (!alive) {
-                    // The path ended: the unit's next sample, or the unit is done.
-                    if (++sample < sample_end) {
+                if (!alive && ++sample < run_end) {
+                    fresh = true;  // the path ended: the run's next sample
+                } else if (!alive) {
+                    // The run's sum joins the pixel's and the next run follows, or,
+                    // in a split job, it is stored for the lane that finishes the pixel.
+                    float4* part = partials + J.part_begin + pixel;
+                    const uint32_t run = (sample - 1u) / J.run_spp;
+                    if (J.units > 1) __stcg(part + (size_t)run * J.pixels, make_float4(sum.x, sum.y, sum.z, 0.0f));
+                    else total = total + sum;
+                    sum = mk(0.0f, 0.0f, 0.0f);
+                    if (J.units == 1 && sample < (uint32_t)J.spp) {
+                        run_end = min(sample + J.run_spp, (uint32_t)J.spp);
                         fresh = true;
                     } else {
                         have = false;
                         bool pixel_done = true;
                         if (J.units > 1) {
-                            // The lane that finishes a pixel's last unit sums them in order.
-                            const uint32_t k = (sample_end - 1u) / J.unit_spp;
-                            float4* part = partials + J.part_begin + pixel;
-                            __stcg(part + (size_t)k * J.pixels, make_float4(sum.x, sum.y, sum.z, 0.0f));
+                            // The lane that finishes a pixel's last run adds them in order
+                            // (rolled: the loops share the instruction cache with the
+                            // walk, and the unrolled one cost 2-4%).
                             __threadfence();
                             pixel_done = atomicAdd(&done_units[J.done_begin + pixel], 1u) + 1u == J.units;
                             if (pixel_done) {
                                 __threadfence();
-                                sum = mk(0.0f, 0.0f, 0.0f);
-                                for (uint32_t q = 0; q < J.units; ++q) sum = sum + f3(__ldcg(part + (size_t)q * J.pixels));
+                                total = mk(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+                                for (uint32_t q = 0; q < J.units; ++q) total = total + f3(__ldcg(part + (size_t)q * J.pixels));
                             }
                         }
                         if (pixel_done) {
                             n_paths += (uint32_t)J.spp;
                             const float inv = 1.0f / (float)J.spp;
-                            J.out[3 * (size_t)pixel + 0] = sum.x * inv;
-                            J.out[3 * (size_t)pixel + 1] = sum.y * inv;
-                            J.out[3 * (size_t)pixel + 2] = sum.z * inv;
+                            J.out[3 * (size_t)pixel + 0] = total.x * inv;
+                            J.out[3 * (size_t)pixel + 1] = total.y * inv;
+                            J.out[3 * (size_t)pixel + 2] = total.z * inv;
                             // Count finished pixels per job (one atomic per job among the lanes
                             // finishing now); the lane that completes a job stamps the clock.
                             const unsigned same = __match_any_sync(__activemask(), job);
@@ -304,9 +314,9 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                         const DevJob& J = jobs[lo];
                         const uint32_t k = (item - first_item[lo]) / J.pixels;
                         pixel = item - first_item[lo] - k * J.pixels;
-                        sample = k * J.unit_spp;
-                        sample_end = min(sample + J.unit_spp, (uint32_t)J.spp);
-                        sum = mk(0.0f, 0.0f, 0.0f);
+                        sample = k * J.run_spp;
+                        run_end = min(sample + J.run_spp, (uint32_t)J.spp);
+                        sum = total = mk(0.0f, 0.0f, 0.0f);
                         have = fresh = true;
                     }
                 }
@@ -562,6 +572,7 @@ void render_batch(aqua_ctx* ctx, const aqua_job* in, size_t n, const aqua_tuning
         d.max_depth = j.max_depth;
         d.rr_depth = 3;
         d.pixels = (uint32_t)j.width * (uint32_t)j.height;
+        d.run_spp = run_spp_of(d.pixels, (uint32_t)j.spp);
     }
     // Shortest job first: the kernel hands out pixels in the order of the
     // device job list, so ordering it by work (pixels x spp) lets small jobs
@@ -621,6 +632,7 @@ void render_persistent(aqua_ctx* ctx, aqua_scene* sc, const aqua_integrator_cfg&
     d.spp = cfg.spp;
     d.max_depth = cfg.max_depth;
     d.rr_depth = cfg.rr_depth;
+    d.run_spp = (uint32_t)cfg.spp;
     d.pixels = (uint32_t)pixels;
     // Whole pixels: one image whose samples run side by side is the wavefront's
     // case.

@@ -175,10 +175,11 @@ struct DevJob {
     uint64_t seed;
     int32_t scene, spp, max_depth, rr_depth;
     uint32_t pixels;         // pixels of the job
-    // A pixel's samples are split into `units` runs of unit_spp (the last one
-    // shorter); unit k of pixel p is work item item_begin + k * pixels + p. With
-    // more than one, the runs' sums go to partials[part_begin + k * pixels + p].
-    uint32_t item_begin, units, unit_spp, part_begin, done_begin;
+    // A pixel's samples are summed in runs of run_spp (the last one shorter), and
+    // the runs' sums in order. A job is one work item per pixel (units = 1) or one
+    // per run: item item_begin + k * pixels + p is run k of pixel p, whose sum goes
+    // to partials[part_begin + k * pixels + p].
+    uint32_t run_spp, item_begin, units, part_begin, done_begin;
 };
 
 // The last batch, kept so an identical batch replays its CUDA graph.
@@ -189,7 +190,7 @@ struct BatchGraph {
     DevScene* d_scenes = nullptr;
     DevJob* d_jobs = nullptr;
     uint32_t* d_counters = nullptr;
-    uint32_t* d_done = nullptr;      // finished units per pixel of the split jobs
+    uint32_t* d_done = nullptr;      // finished runs per pixel of the split jobs
     float4* d_partials = nullptr;
     unsigned long long* d_clocks = nullptr;
     unsigned long long* d_stats = nullptr;

@@ -405,7 +405,9 @@ AQUA_API aqua_status aqua_autotune(aqua_ctx* ctx, aqua_scene* scene,
  * them one path after another; idle lanes take the next ones from a global
  * queue on which the jobs are laid out shortest first (pixels x spp), so small
  * jobs complete early. Every job's image
- * equals aqua_render's. rgb_out of each job is a device buffer. stats->job_ms,
+ * equals aqua_render's up to the order in which FP32 sums are taken, and has
+ * the same bits whatever the other jobs, the launch shape and the GPU are.
+ * rgb_out of each job is a device buffer. stats->job_ms,
  * when non-NULL, receives each job's completion time from the start of the
  * launch (device clock). tuning->block_trace = threads per block (64, 128,
  * 256), tuning->blocks_per_sm = persistent blocks per SM (0 = occupancy). */
