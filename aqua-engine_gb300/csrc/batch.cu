@@ -441,14 +441,9 @@ static BatchResult launch_jobs(aqua_ctx* ctx, std::vector<DevJob>& jobs, std::ve
     BatchGraph& g = ctx->batch;
     uint32_t parts = 0, split_pixels = 0;
     uint32_t items = split_jobs(jobs, (uint64_t)ctx->num_sms * kBatchLanes, split, split_pixels, parts);
-    bool reuse = same_batch(g, jobs, scenes, block, grid) && tune.use_graph != 0;
-    if (!reuse && split && g.exec && tune.use_graph != 0) {
-        // The last batch may have had to run unsplit (below).
-        std::vector<DevJob> whole = jobs;
-        uint32_t a = 0, b = 0;
-        split_jobs(whole, 1, false, a, b);
-        reuse = same_batch(g, whole, scenes, block, grid);
-    }
+    // A batch that ran whole for want of memory is not the one asked for: it is
+    // built anew, and split if there is room by then.
+    const bool reuse = same_batch(g, jobs, scenes, block, grid) && tune.use_graph != 0;
     if (!reuse) {
         batch_release(ctx);
         size_t off = 0;
