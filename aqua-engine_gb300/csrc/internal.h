@@ -131,7 +131,8 @@ struct NrcNet {
     uint2* frag_inf = nullptr;  // forward fragments of the inference weights
     uint8_t* img_tc = nullptr;  // inference weights in the tcgen05 shared-memory layout
     uint8_t* img_tc_w = nullptr;  // the trained weights w in that layout (training)
-    uint32_t* tc_err = nullptr; // set by the tcgen05 kernel when a wait expired
+    uint32_t* tc_err = nullptr; // set by a tcgen05 kernel when a wait expired; steps after it change nothing
+    uint32_t* tc_applied = nullptr;  // number of the last step that Adam applied (tcgen05)
     int forward_tc = 0;         // 1: inference runs on tcgen05 (else mma.sync)
     float ema_decay = 0.0f;  // 0 = inference uses w itself
     DevBuf train;            // training scratch, sized by train_rows
@@ -241,7 +242,7 @@ struct aqua_ctx {
     // pageable memory is staged by the driver and waits for it.
     unsigned int* pinned_counter = nullptr;  // 16 queue counts
     unsigned long long* pinned_stats = nullptr;  // 16 statistics
-    double* pinned_loss = nullptr;           // the training loss and, after it, the tcgen05 error flag
+    double* pinned_loss = nullptr;           // the training loss, the tcgen05 error flag and the last step applied
     std::unique_ptr<aq::EventPair> timer;    // timing of one stretch of the stream, created on first use
     std::map<std::pair<const void*, int>, int> resident;  // occupancy by kernel and block size
     std::vector<cudaEvent_t> events;         // pool for stage timing

@@ -318,19 +318,23 @@ __global__ void __launch_bounds__(128) k_nrc_wgrad(const uint32_t* __restrict__ 
 // of loads, 8 us at 64 partials.) losses, when given, are summed by block 0
 // into *loss. With img_w non-null the new weights also go straight into the
 // tcgen05 weight images (of w and of the inference weights), so no packing
-// launch follows the step.
+// launch follows the step. With err given and set, a kernel before gave up
+// waiting and the partials are not all there: nothing is changed. Otherwise
+// *applied becomes the step's number.
 constexpr int kAdamWarps = 8;
 
 __global__ void __launch_bounds__(32 * kAdamWarps)
     k_nrc_adam(const float* __restrict__ partial, int chunks, float* __restrict__ w, float* __restrict__ m,
                float* __restrict__ v, float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1,
                float c2, float* __restrict__ ema, float ema_decay, uint8_t* __restrict__ img_w,
-               uint8_t* __restrict__ img_inf, const double* __restrict__ losses, double* __restrict__ loss) {
+               uint8_t* __restrict__ img_inf, const double* __restrict__ losses, double* __restrict__ loss,
+               const uint32_t* __restrict__ err, uint32_t* __restrict__ applied, uint32_t step) {
     __shared__ float s_sum[kAdamWarps][32];
     grid_dep_wait();
     grid_dep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p = (int)blockIdx.x * 32 + lane;
+    const bool failed = err && __ldcg(err) != 0u;
     float part = 0.0f;
     if (p < kNrcParams)
         for (int k = warp; k < chunks; k += kAdamWarps) part += __ldcg(partial + (size_t)k * kNrcParams + p);
@@ -339,10 +343,10 @@ __global__ void __launch_bounds__(32 * kAdamWarps)
         double sum = 0.0;
         for (int k = lane; k < chunks; k += 32) sum += __ldcg(losses + k);
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-        if (lane == 0) *loss = sum;
+        if (lane == 0 && !failed) *loss = sum, *applied = step;
     }
     __syncthreads();
-    if (warp != 0 || p >= kNrcParams) return;
+    if (warp != 0 || p >= kNrcParams || failed) return;
     float g = 0.0f;
 #pragma unroll
     for (int j = 0; j < kAdamWarps; ++j) g += s_sum[j][lane];
@@ -487,8 +491,10 @@ void nrc_alloc(aqua_ctx* ctx, NrcNet& net) {
     net.frag_inf = (uint2*)(b + o_fi);
     net.img_tc = (uint8_t*)(b + o_tc);
     net.img_tc_w = (uint8_t*)(b + o_tw);
-    net.tc_err = (uint32_t*)(b + o_l + 8);  // next to the loss: one read-back carries both
-    AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 4, ctx->stream));
+    // Next to the loss: one read-back carries all three.
+    net.tc_err = (uint32_t*)(b + o_l + 8);
+    net.tc_applied = net.tc_err + 1;
+    AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 8, ctx->stream));
 }
 
 void nrc_release(NrcNet& net) {
@@ -532,6 +538,7 @@ void nrc_set_weights(aqua_ctx* ctx, NrcNet& net, const float* host_w) {
     AQ_CUDA(cudaMemsetAsync(net.v, 0, 4 * kNrcParams, ctx->stream));
     AQ_CUDA(cudaMemsetAsync(net.grad, 0, 4 * kNrcParams, ctx->stream));
     AQ_CUDA(cudaMemcpyAsync(net.ema, net.w, 4 * kNrcParams, cudaMemcpyDeviceToDevice, ctx->stream));
+    AQ_CUDA(cudaMemsetAsync(net.tc_applied, 0, 4, ctx->stream));
     net.step = 0;
     nrc_pack(ctx, net);
     AQ_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -602,7 +609,8 @@ void nrc_train_step_dev(aqua_ctx* ctx, NrcNet& net, const uint16_t* X, const flo
     launch_chained(k_nrc_adam, dim3((kNrcParams + 31) / 32), dim3(32 * kAdamWarps), 0, st, (const float*)net.partial,
                    chunks, net.w, net.m, net.v, net.grad, net.lr, net.beta1, net.beta2, net.eps, c1, c2, net.ema,
                    net.ema_decay, net.forward_tc ? net.img_tc_w : nullptr, net.img_tc,
-                   net.forward_tc ? (const double*)net.losses : nullptr, net.loss);
+                   net.forward_tc ? (const double*)net.losses : nullptr, net.loss,
+                   net.forward_tc ? (const uint32_t*)net.tc_err : nullptr, net.tc_applied, (uint32_t)net.step);
     if (!net.forward_tc) nrc_pack_frags(ctx, net);
     AQ_CUDA(cudaGetLastError());
     net.launches += net.forward_tc ? 2 : 6;
@@ -613,9 +621,10 @@ void nrc_read_back(aqua_ctx* ctx, NrcNet& net) {
 }
 
 void nrc_check_tc(aqua_ctx* ctx, NrcNet& net) {
-    uint32_t e;
-    memcpy(&e, ctx->pinned_loss + 1, 4);
-    if (!net.forward_tc || !e) return;
+    uint32_t e[2];  // the flag, the last step applied
+    memcpy(e, ctx->pinned_loss + 1, 8);
+    if (!net.forward_tc || !e[0]) return;
+    net.step -= (int64_t)((uint32_t)net.step - e[1]);  // steps that changed nothing were not taken
     AQ_CUDA(cudaMemsetAsync(net.tc_err, 0, 4, ctx->stream));
     throw Error(AQUA_ERR_TIMEOUT, "tensor-core kernel: a completion wait expired");
 }
