@@ -70,6 +70,7 @@ static void free_staging(aqua_scene* s) {
 
 void scene_release(aqua_scene* s) {
     dev_free(s->dev);
+    dev_free(s->walk);
     free_staging(s);
 }
 
@@ -104,7 +105,7 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     for (const aqua_material& m : h.mats)
         if (m.specular_tint > 0.0f || m.sheen > 0.0f || m.clearcoat > 0.0f || m.transmission > 0.0f) full_bsdf = true;
     size_t total = align256(o_mext + (full_bsdf ? 32 * h.mats.size() : 0));
-    // Walk nodes follow the uploaded image; the device derives them.
+    // Walk nodes, which the device derives from the uploaded image.
     bool use_walk = !use_q && nn >= kWalkNodesFrom && walk_stack_fits(s->bvh) && !ctx->host_only;
     for (int a = 0; a < 3; ++a)  // a walk node's frame must stay within the float range
         use_walk = use_walk && std::fabs(s->bvh.lo[a]) < 1e15f && std::fabs(s->bvh.hi[a]) < 1e15f;
@@ -183,11 +184,20 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     s->bvh_format_used = use_q ? AQUA_BVH_QUANTIZED : AQUA_BVH_FULL;
     if (ctx->host_only) return;  // host-only context: no device image
     dev_free(s->dev);
-    dev_alloc(ctx, s->dev, total + (use_walk ? sizeof(float) * kBvhQNodeFloats * nn : 0));
+    dev_free(s->walk);
+    dev_alloc(ctx, s->dev, total);
+    if (use_walk) {
+        try {
+            dev_alloc(ctx, s->walk, sizeof(float) * kBvhQNodeFloats * nn);
+        } catch (const Error& e) {
+            if (e.status != AQUA_ERR_OOM) throw;
+            use_walk = false;  // no room: the scene is walked through its full-precision nodes
+        }
+    }
     char* d = (char*)s->dev.ptr;
     DevScene& ds = s->ds;
     ds.nodes = (const float4*)(d + o_nodes);
-    ds.wnodes = use_walk ? (const float4*)(d + total) : nullptr;
+    ds.wnodes = use_walk ? (const float4*)s->walk.ptr : nullptr;
     ds.qbvh = use_q ? 1 : 0;
     ds.tris = (const float4*)(d + o_tris);
     ds.uvs = (const float2*)(d + o_uvs);
@@ -209,7 +219,7 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
         // The load ends with the nodes in place: any context may walk them next,
         // on a stream that does not wait for this one.
         s->uploaded = false;
-        build_walk_nodes(ctx, ds, (float4*)(d + total));
+        build_walk_nodes(ctx, ds, (float4*)s->walk.ptr);
         AQ_CUDA(cudaStreamSynchronize(ctx->stream));
         s->uploaded = true;
     }
@@ -455,7 +465,7 @@ AQUA_API aqua_status aqua_scene_get_info(aqua_ctx* ctx, const aqua_scene* s, aqu
         out->num_bvh_nodes = s->bvh.num_nodes();
         out->bvh_depth = s->bvh.depth;
         out->max_leaf_size = s->bvh.max_leaf;
-        out->device_bytes = s->dev.bytes;
+        out->device_bytes = s->dev.bytes + s->walk.bytes;
         out->upload_bytes = s->bytes;
         for (int i = 0; i < 3; ++i) out->env[i] = s->host.env[i];
         out->bvh_format = s->bvh_format_used;

@@ -216,7 +216,8 @@ struct aqua_scene {
     bool pinned_is_cuda = false;
     size_t bytes = 0;          // bytes of the device image
     aq::DevBuf dev;            // device copy
-    aq::DevScene ds{};         // pointers into dev
+    aq::DevBuf walk;           // walk nodes of large trees
+    aq::DevScene ds{};         // pointers into dev and walk
     bool uploaded = false;
 };
 
