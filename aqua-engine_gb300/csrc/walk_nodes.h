@@ -17,10 +17,18 @@
 
 namespace aq {
 
-// One axis of a walk node from the child planes lo[c], hi[c] and the links. All
-// steps are exact: a plane lo + q 2^e of floats lo and 8-bit q needs at most 41
-// bits (2^e is at least an 256th of an ulp of the larger plane), so the
-// doubles below hold it.
+// a - b = diff + the returned rest, exactly (Knuth's two-sum; no overflow here).
+AQ_HD double diff_exact(double a, double b, double& diff) {
+    diff = a - b;
+    const double t = diff - a;
+    return (a - (diff - t)) - (b + t);
+}
+
+// One axis of a walk node from the child planes lo[c], hi[c] and the links: the
+// decoded planes origin + q s bound the children's exactly. A difference of two
+// floats need not fit a double, but its rounding can only hide that it lies just
+// below or above a multiple of the step, which the rest shows. (Products with and
+// quotients by a power of two are exact.)
 AQ_HD void walk_axis(const float* plo, const float* phi, const int32_t* link, float& origin, float& step,
                      uint32_t& lo_bytes, uint32_t& hi_bytes) {
     float lo = INFINITY, hi = -INFINITY;
@@ -31,10 +39,13 @@ AQ_HD void walk_axis(const float* plo, const float* phi, const int32_t* link, fl
         }
     if (!(lo <= hi)) lo = hi = 0.0f;  // no children (not produced by the builder)
     int e = -100;
+    double d, rest;
     if (hi > lo) {  // smallest step whose 255 multiples reach hi
-        const int k = ilogb(((double)hi - (double)lo) / 255.0);
+        rest = diff_exact(hi, lo, d);
+        const int k = ilogb(d / 255.0);
         e = k > -100 ? k : -100;
-        if (ldexp(255.0, e) < (double)hi - (double)lo) ++e;
+        const double reach = ldexp(255.0, e);
+        if (reach < d || (reach == d && rest > 0.0)) ++e;
     }
     const double s = ldexp(1.0, e);
     origin = lo;
@@ -43,8 +54,12 @@ AQ_HD void walk_axis(const float* plo, const float* phi, const int32_t* link, fl
     for (int c = 0; c < 4; ++c) {
         uint32_t ql = 255, qh = 0;  // empty slot: an inverted box
         if (link[c] != ~0) {
-            ql = (uint32_t)floor(((double)plo[c] - (double)lo) / s);
-            qh = (uint32_t)ceil(((double)phi[c] - (double)lo) / s);
+            rest = diff_exact(plo[c], lo, d);
+            ql = (uint32_t)floor(d / s);
+            if (rest < 0.0 && (double)ql * s == d) --ql;
+            rest = diff_exact(phi[c], lo, d);
+            qh = (uint32_t)ceil(d / s);
+            if (rest > 0.0 && (double)qh * s == d) ++qh;
         }
         lo_bytes |= ql << (8 * c);
         hi_bytes |= qh << (8 * c);
@@ -75,10 +90,10 @@ AQ_HD float walk_byte(uint32_t word, int k) {
 //   (1 + q 2^-15) A + (b - A) = b + q s / d.
 // The rounding errors of a plane's distance stay below
 // 5 x 2^-24 (|b| + |A|); near planes are moved back and far planes forward
-// by 8 x 2^-24 (|b| + |A|) (1/64 of a step at most), which also covers the
-// rounding of slab_entry on the exact planes. So every box that slab_entry
-// accepts is accepted here, and a walk whose hits are
-// confirmed (walk_confirmed) finds what the full-precision walk finds. An
+// by 8 x 2^-24 (|b| + |A|) (1/64 of a step at least, more from far away), which
+// also covers the rounding of slab_entry on the exact planes. So every box that
+// slab_entry accepts is accepted here, at no later distance, and a walk whose hits
+// are confirmed (walk_confirmed) finds what the full-precision walk finds. An
 // empty slot is accepted too where the node is flat or the ray's origin lies
 // some 10^5 node extents away: its leaf holds no triangle, but the walk may
 // push all four slots of a node (walk_stack_fits).
