@@ -474,7 +474,7 @@ __device__ __forceinline__ void traverse_lanes(const DevScene& S, uint32_t n, ui
             }
         }
         if (node == kTraversalDone) {
-                        if (NODES == kNodesWalk && !walk_confirmed(S, rp, r)) walk_full(S, rp, sh, any, stack, r);
+            if (NODES == kNodesWalk && !walk_confirmed(S, rp, r)) walk_full(S, rp, sh, any, stack, r);
             done(tag, r);
             have = false;
         }

@@ -258,11 +258,14 @@ namespace aq {
 
 // Trees of at least this many nodes are walked through walk nodes. A smaller
 // tree's full-precision nodes are served by L1 and L2 well enough that the
-// walk is bound by instruction issue, and the tighter boxes win; rooms of
-// tessellated spheres, 512 x 512 at 16 spp and 1M random rays, full against
-// walk nodes: 8 nodes (Cornell GGX 1024^2, 64 spp) 38.4 / 45.2 ms; 6.0k nodes
+// walk is bound by instruction issue, and the tighter boxes win. Full against walk
+// nodes, rooms of tessellated spheres at 512 x 512 and 16 spp, and 1M random rays in
+// them: 8 nodes (Cornell GGX 1024^2, 64 spp) 38.4 / 45.2 ms; 6.0k nodes
 // 3.57 / 3.77 ms and 188 / 192 us; 33k 4.32 / 4.41 ms and 228 / 231 us; 131k
-// 4.82 / 4.87 ms and 260 / 252 us; the interior's 294k 47.9 / 40.8 ms.
+// 4.82 / 4.87 ms and 260 / 252 us; 160k 4.04 / 4.06 ms and 249 / 218 us; 162k 5.15 /
+// 4.74 ms and 310 / 267 us; 167k 5.85 / 5.32 ms and 506 / 426 us; 196k 5.62 / 5.00 ms
+// and 339 / 289 us; 260k 6.16 / 5.37 ms and 405 / 329 us; the interior's 294k 47.9 /
+// 40.8 ms.
 constexpr size_t kWalkNodesFrom = 150000;
 
 inline EventPair& timer(aqua_ctx* ctx) {
