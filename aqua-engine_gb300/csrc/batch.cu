@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
     bool have = false, walking = false, drained = false;
     int job = 0;
     uint32_t pixel = 0, sample = 0, run_end = 0;
-    v3 sum = mk(0.0f, 0.0f, 0.0f), total = mk(0.0f, 0.0f, 0.0f);  // of the run; of an unsplit pixel's runs before
+    v3 sum = mk(0.0f, 0.0f, 0.0f);  // of the run
     LanePath P;
     P.shadow = false;
     // The ray in flight.
@@ -249,14 +249,17 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                 if (!alive && ++sample < run_end) {
                     fresh = true;  // the path ended: the run's next sample
                 } else if (!alive) {
-                    // The run's sum joins the pixel's and the next run follows, or,
-                    // in a split job, it is stored for the lane that finishes the pixel.
+                    // The run's sum joins the pixel's in the film and the next run follows
+                    // (the registers of a second sum in the lane cost 1%), or, in a split
+                    // job, it is stored for the lane that finishes the pixel.
                     float4* part = partials + J.part_begin + pixel;
                     const uint32_t run = (sample - 1u) / J.run_spp;
+                    float* out = J.out + 3 * (size_t)pixel;
                     if (J.units > 1) __stcg(part + (size_t)run * J.pixels, make_float4(sum.x, sum.y, sum.z, 0.0f));
-                    else total = total + sum;
-                    sum = mk(0.0f, 0.0f, 0.0f);
+                    else if (run != 0u) sum = mk(__ldcg(out), __ldcg(out + 1), __ldcg(out + 2)) + sum;
                     if (J.units == 1 && sample < (uint32_t)J.spp) {
+                        out[0] = sum.x, out[1] = sum.y, out[2] = sum.z;
+                        sum = mk(0.0f, 0.0f, 0.0f);
                         run_end = min(sample + J.run_spp, (uint32_t)J.spp);
                         fresh = true;
                     } else {
@@ -270,17 +273,17 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                             pixel_done = atomicAdd(&done_units[J.done_begin + pixel], 1u) + 1u == J.units;
                             if (pixel_done) {
                                 __threadfence();
-                                total = mk(0.0f, 0.0f, 0.0f);
+                                sum = mk(0.0f, 0.0f, 0.0f);
 #pragma unroll 1
-                                for (uint32_t q = 0; q < J.units; ++q) total = total + f3(__ldcg(part + (size_t)q * J.pixels));
+                                for (uint32_t q = 0; q < J.units; ++q) sum = sum + f3(__ldcg(part + (size_t)q * J.pixels));
                             }
                         }
                         if (pixel_done) {
                             n_paths += (uint32_t)J.spp;
                             const float inv = 1.0f / (float)J.spp;
-                            J.out[3 * (size_t)pixel + 0] = total.x * inv;
-                            J.out[3 * (size_t)pixel + 1] = total.y * inv;
-                            J.out[3 * (size_t)pixel + 2] = total.z * inv;
+                            out[0] = sum.x * inv;
+                            out[1] = sum.y * inv;
+                            out[2] = sum.z * inv;
                             // Count finished pixels per job (one atomic per job among the lanes
                             // finishing now); the lane that completes a job stamps the clock.
                             const unsigned same = __match_any_sync(__activemask(), job);
@@ -316,7 +319,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                         pixel = item - first_item[lo] - k * J.pixels;
                         sample = k * J.run_spp;
                         run_end = min(sample + J.run_spp, (uint32_t)J.spp);
-                        sum = total = mk(0.0f, 0.0f, 0.0f);
+                        sum = mk(0.0f, 0.0f, 0.0f);
                         have = fresh = true;
                     }
                 }

@@ -29,13 +29,14 @@ inline uint32_t run_spp_of(uint32_t pixels, uint32_t spp) {
 // pixels of a small batch kept a few lanes busy long after the others had
 // run dry (a 51 x 145 view of the interior at 43 spp took 19 ms alone). A job is
 // split when its pixels hold more samples than a kShares-th of the paths that a
-// lane runs in the whole batch (four views of up to 128^2 at 6 spp 2.41 -> 0.72 ms, ten of up to
-// 300^2 at 16 spp 7.56 -> 2.42, twenty of up to 512^2 at 48 spp 41.4 -> 33.7). A
+// lane runs in the whole batch (four views of up to 128^2 at 6 spp 2.41 -> 0.70 ms, ten of up to
+// 300^2 at 16 spp 7.56 -> 2.42, twenty of up to 512^2 at 48 spp 41.4 -> 33.3). A
 // large batch keeps whole pixels, and so do more and more jobs of one whose items
 // would not fit 32 bits or whose stored runs would take more than 1 GB.
 // Returns the items; pixels and stored runs of the split jobs by reference.
 constexpr uint64_t kBatchLanes = 768;  // per SM
-constexpr uint64_t kShares = 64;       // 16, 32 and 128: within 4%
+constexpr uint64_t kShares = 64;       // 16, 32, 128: 34.2, 33.4, 33.4 ms for the twenty views; 64 views at 64 spp
+                                       // 190, 180, 175 ms against 177; others within 1%
 constexpr uint64_t kMaxStoredRuns = (uint64_t)1 << 26;
 
 template <class Job>
