@@ -543,6 +543,7 @@ void render_batch(aqua_ctx* ctx, const aqua_job* in, size_t n, const aqua_tuning
     for (size_t i = 0; i < n; ++i) {
         const aqua_job& j = in[i];
         if (!j.scene || !j.rgb_out) throw Error(AQUA_ERR_INVALID_ARG, "job " + std::to_string(i) + ": scene and rgb_out must be non-NULL");
+        if (!j.scene->uploaded) throw Error(AQUA_ERR_INVALID_ARG, "job " + std::to_string(i) + ": the scene has no device image");
         if (j.width <= 0 || j.height <= 0 || j.width > 16384 || j.height > 16384)
             throw Error(AQUA_ERR_INVALID_ARG, "job " + std::to_string(i) + ": resolution out of range");
         if (j.spp <= 0 || j.max_depth < 0 || j.max_depth > 250)

@@ -183,6 +183,7 @@ void scene_build_device(aqua_ctx* ctx, aqua_scene* s, bool rebuild_bvh) {
     s->bytes = total;
     s->bvh_format_used = use_q ? AQUA_BVH_QUANTIZED : AQUA_BVH_FULL;
     if (ctx->host_only) return;  // host-only context: no device image
+    s->uploaded = false;  // until the new image is complete
     dev_free(s->dev);
     dev_free(s->walk);
     dev_alloc(ctx, s->dev, total);
@@ -300,6 +301,10 @@ static aqua_status guard(aqua_ctx* ctx, F&& f) {
 static void need(bool c, const char* msg) {
     if (!c) throw Error(AQUA_ERR_INVALID_ARG, msg);
 }
+
+// A scene from a host-only context, or one whose image could not be rebuilt
+// (aqua_scene_set_bvh_format out of memory), has nothing on the device.
+static void need_image(const aqua_scene* s) { need(s->uploaded, "the scene has no device image"); }
 
 static void need_device(aqua_ctx* ctx) {
     if (ctx->host_only) throw Error(AQUA_ERR_UNSUPPORTED, "this call needs a CUDA device; the context is host-only");
@@ -631,6 +636,7 @@ AQUA_API aqua_status aqua_trace(aqua_ctx* ctx, aqua_scene* s, const aqua_ray* ra
         need_device(ctx);
         need(n == 0 || (rays && out), "rays and out must be non-NULL");
         need(n < ((size_t)1 << 34), "too many rays");
+        if (n > 0) need_image(s);
         trace_rays(ctx, s, rays, n, out, flags, counts);
     });
 }
@@ -640,6 +646,7 @@ AQUA_API aqua_status aqua_render(aqua_ctx* ctx, aqua_scene* s, const aqua_integr
     return guard(ctx, [&]() {
         need(s && cfg && rgb_out, "scene, cfg and rgb_out must be non-NULL");
         need_device(ctx);
+        need_image(s);
         aqua_tuning t;
         if (tuning) t = *tuning;
         else aqua_tuning_defaults(&t);
@@ -663,6 +670,7 @@ AQUA_API aqua_status aqua_autotune(aqua_ctx* ctx, aqua_scene* s, const aqua_inte
     return guard(ctx, [&]() {
         need(s && cfg && out, "scene, cfg and out must be non-NULL");
         need_device(ctx);
+        need_image(s);
         if (cfg->type != AQUA_INTEGRATOR_PATH)
             throw Error(AQUA_ERR_UNSUPPORTED, "the autotuner tunes the path integrator");
         aqua_integrator_cfg c = *cfg;
@@ -780,6 +788,7 @@ AQUA_API aqua_status aqua_render_noalloc(aqua_ctx* ctx, aqua_scene* s, const aqu
     return guard(ctx, [&]() {
         need(s && cfg && rgb_out_device, "scene, cfg and rgb_out_device must be non-NULL");
         need_device(ctx);
+        need_image(s);
         if (cfg->type != AQUA_INTEGRATOR_PATH)
             throw Error(AQUA_ERR_UNSUPPORTED, "aqua_render_noalloc renders the path integrator only");
         render_noalloc(ctx, s, *cfg, rgb_out_device, stats);
@@ -948,6 +957,7 @@ AQUA_API aqua_status aqua_render_nrc(aqua_ctx* ctx, aqua_scene* s, const aqua_in
     return guard(ctx, [&]() {
         need(s && cfg && nrc && rgb_out, "scene, cfg, nrc and rgb_out must be non-NULL");
         need_device(ctx);
+        need_image(s);
         aqua_tuning t;
         if (tuning) t = *tuning;
         else aqua_tuning_defaults(&t);
