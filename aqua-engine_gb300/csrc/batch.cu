@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
     int job = 0;
     uint32_t pixel = 0, sample = 0, run_end = 0;
     v3 sum = mk(0.0f, 0.0f, 0.0f);  // of the run
+    volatile float rest[3];  // of a whole pixel's runs before: kept out of the registers
     LanePath P;
     P.shadow = false;
     // The ray in flight.
@@ -249,16 +250,15 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                 if (!alive && ++sample < run_end) {
                     fresh = true;  // the path ended: the run's next sample
                 } else if (!alive) {
-                    // The run's sum joins the pixel's in the film and the next run follows
-                    // (the registers of a second sum in the lane cost 1%), or, in a split
-                    // job, it is stored for the lane that finishes the pixel.
+                    // The run's sum joins the pixel's and the next run follows (with that
+                    // sum in registers the 64-job batch took 1% longer), or, in a split job,
+                    // it is stored for the lane that finishes the pixel.
                     float4* part = partials + J.part_begin + pixel;
                     const uint32_t run = (sample - 1u) / J.run_spp;
-                    float* out = J.out + 3 * (size_t)pixel;
                     if (J.units > 1) __stcg(part + (size_t)run * J.pixels, make_float4(sum.x, sum.y, sum.z, 0.0f));
-                    else if (run != 0u) sum = mk(__ldcg(out), __ldcg(out + 1), __ldcg(out + 2)) + sum;
+                    else if (run != 0u) sum = mk(rest[0], rest[1], rest[2]) + sum;
                     if (J.units == 1 && sample < (uint32_t)J.spp) {
-                        out[0] = sum.x, out[1] = sum.y, out[2] = sum.z;
+                        rest[0] = sum.x, rest[1] = sum.y, rest[2] = sum.z;
                         sum = mk(0.0f, 0.0f, 0.0f);
                         run_end = min(sample + J.run_spp, (uint32_t)J.spp);
                         fresh = true;
@@ -281,9 +281,9 @@ __global__ void __launch_bounds__(256, 3) k_batch(const DevScene* __restrict__ s
                         if (pixel_done) {
                             n_paths += (uint32_t)J.spp;
                             const float inv = 1.0f / (float)J.spp;
-                            out[0] = sum.x * inv;
-                            out[1] = sum.y * inv;
-                            out[2] = sum.z * inv;
+                            J.out[3 * (size_t)pixel + 0] = sum.x * inv;
+                            J.out[3 * (size_t)pixel + 1] = sum.y * inv;
+                            J.out[3 * (size_t)pixel + 2] = sum.z * inv;
                             // Count finished pixels per job (one atomic per job among the lanes
                             // finishing now); the lane that completes a job stamps the clock.
                             const unsigned same = __match_any_sync(__activemask(), job);

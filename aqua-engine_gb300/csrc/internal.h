@@ -192,7 +192,7 @@ struct BatchGraph {
     DevJob* d_jobs = nullptr;
     uint32_t* d_counters = nullptr;
     uint32_t* d_done = nullptr;      // finished runs per pixel of the split jobs
-    float4* d_partials = nullptr;
+    float4* d_partials = nullptr;    // the runs' sums of the split jobs
     unsigned long long* d_clocks = nullptr;
     unsigned long long* d_stats = nullptr;
     std::vector<DevJob> jobs;

@@ -36,6 +36,16 @@ def test_a_job_has_the_same_bits_in_any_company(gpu_ctx):
     for other in COMPANY:
         for a, b in zip(alone, render(JOBS + [other])):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    # Jobs that share a film (the same view twice) leave the view's image in it.
+    film = torch.full((200, 300, 3), -1.0, device="cuda")
+    rest = torch.zeros((2048, 2048, 3), device="cuda")
+    torch.cuda.synchronize()
+    twice = [(scenes[c], w, h, spp, depth, seed, film.data_ptr()) for (c, w, h, spp, depth, seed) in [JOBS[-1]] * 2]
+    for company in ([], [(scenes[1], 2048, 2048, 120, 1, 9, rest.data_ptr())]):
+        film.fill_(-1.0)
+        torch.cuda.synchronize()
+        gpu_ctx.render_batch(twice + company)
+        assert np.array_equal(film.cpu().numpy().view(np.uint32), alone[-1].view(np.uint32))
     for (c, w, h, spp, depth, seed), img in zip(JOBS, alone):
         s = scenes[c]
         s.set_resolution(w, h)
